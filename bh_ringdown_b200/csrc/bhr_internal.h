@@ -163,6 +163,43 @@ cudaError_t encode_strip_maps(double *state, double *ctab, int N, int M, StripMa
 // (a.out) on the interior; u1 stays in shared memory.
 cudaError_t launch_stage12_strip(const StripMaps &maps, const StageArgs &a, cudaStream_t st, bool pdl = true);
 
+// Whole steps of a small grid in one cooperative launch (bhr_resident.cu):
+// one 64-column tile of up to kResidentMaxRows rows per block, strips x segs
+// blocks.  ok is false for grids that do not fit (more strips than SMs, or
+// taller tiles).
+constexpr int kResidentMaxRows = 32;
+constexpr int kResidentChunk = 64;  // steps per launch
+struct ResidentGeom {
+  int strips, segs, rmax;
+  bool ok;
+};
+ResidentGeom resident_geometry(int N, int M);
+size_t resident_inbox_bytes(const ResidentGeom &g);
+struct ResidentArgs {
+  double *u;             // state planes, advanced in place
+  const double *coltab, *rowtab, *bb;
+  ulonglong2 *inbox;     // resident_inbox_bytes, no word numbered seq .. seq + 3 steps - 1 yet
+  int *err;
+  double *hist;          // [steps][2][2][M]: psi_re, psi_im at columns ext[0], ext[1], or nullptr
+  unsigned long long seq;  // number of the first stage's edge words
+  int N, M, even_m, strips, segs, rmax, steps;
+  int ext[2];            // columns recorded (-1: none)
+  int close;             // 1: also write the closure of the boundary rows and columns
+  double dt, cx, cy, cyy, cko, a2, m4a;
+};
+// Extraction of a resident launch's steps: snapshots of the time integrals
+// on output steps [kResidentChunk][4][M]; count: {first row, rows}.
+struct ChunkArgs {
+  ExtractArgs E;
+  double *hist;          // its closure points are filled in
+  double *snap;
+  int *count;
+  int steps;
+};
+cudaError_t launch_resident(const ResidentArgs &a, cudaStream_t st);
+cudaError_t launch_chunk_extract(const ChunkArgs &a, cudaStream_t st);
+cudaError_t prepare_resident_kernels();
+
 // Mixed precision (BHR_MIXED): SSP-RK3 rearranged so that FP32 carries only
 // O(dt^2) corrections.  With delta1 = dt L(u^n) (L with the source) and L0
 // the homogeneous operator,
@@ -235,7 +272,8 @@ enum StageTiling {
   kTilingPersistent = 2,
   kTilingBlock8n = 3,
   kTilingRing = 4,
-  kTilingStrip12 = 5  // stages 1 and 2 fused (launch_stage12_strip), stage 3 as block8n
+  kTilingStrip12 = 5,  // stages 1 and 2 fused (launch_stage12_strip), stage 3 as block8n
+  kTilingResident = 6  // whole steps in one launch (launch_resident)
 };
 constexpr int tiling_rows(int tiling) {
   return (tiling == kTilingBlock8 || tiling == kTilingBlock8n || tiling == kTilingRing) ? 8 : 16;

@@ -1534,6 +1534,7 @@ cudaError_t prepare_kernels() {
   const int s8 = static_cast<int>(sizeof(StageSmem<8>) + 128), s16 = static_cast<int>(sizeof(StageSmem<16>) + 128);
   const int sp = static_cast<int>(persist_smem_bytes()), sr = static_cast<int>(ring_smem_bytes());
   constexpr auto kSmem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if (cudaError_t r = prepare_resident_kernels()) return r;
   if (cudaError_t r = cudaFuncSetAttribute(stage12_strip_kernel, kSmem, static_cast<int>(strip_smem_bytes()))) return r;
   for (int stage = 1; stage <= 5; stage++) {
     const cudaError_t e = by_stage(stage, [&](auto sc) {

@@ -9,7 +9,10 @@
 // memory it already owns, and the two intermediate SSP-RK3 stages plus the
 // coefficient tables live in one file-scope __device__ array of fixed size
 // below (every GPU that loads the library holds it until the process
-// exits).  The stage kernels are the same ones bhr_solver_step launches.
+// exits).  The kernels are the same ones bhr_solver_step launches: all steps
+// of the call in one cooperative launch where the grid fits one tile per
+// SM (the array's stage part then holds the tiles' edge words), stage kernels
+// otherwise.
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -38,6 +41,7 @@ constexpr size_t kScratchDoubles = kFlagOff + 32;  // about 11.2 MB in all
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
 constexpr int kMaxDevices = 64;
+constexpr int kNoAllocLaunchSteps = 4096;  // steps per resident launch
 
 // What one device's scratch holds: the parameters its tables were built
 // for and the tensor maps over the last state it stepped.  Rebuilding the
@@ -50,6 +54,10 @@ struct DeviceScratch {
   double Xmin = 0, Xmax = 0, mass = 0, a = 0, m = 0, dt = 0;
   double *state = nullptr;
   StageMaps maps[3];
+  // The stage part holds edge words of resident launches, numbered below seq.
+  bool inbox_valid = false;
+  unsigned long long seq = 1;
+  bool flag_clear = false;  // the error flag is known to be zero
 };
 
 std::mutex g_mu;
@@ -126,7 +134,9 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
   const int N = p->N, M = p->M;
   const double dx = (p->Xmax - p->Xmin) / N, dth = kPiParm / M;
   const bool rebuild = !same_tables(D, *p);
-  if (rebuild || D.state != state) {
+  const ResidentGeom geom = resident_geometry(N, M);
+  bool resident = geom.ok && resident_inbox_bytes(geom) <= 2 * kStageDoubles * sizeof(double);
+  auto encode = [&]() -> int {
     for (int i = 0; i < 3; i++) {
       double *bufs[3] = {state, u1, u2};
       StageMaps &mp = D.maps[i];
@@ -140,11 +150,13 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
       }
     }
     D.state = state;
-  }
+    return BHR_OK;
+  };
   if (rebuild) {
     // The tables are rewritten while no kernel of an earlier call may still
     // read them: every call ends with its stream drained.
     D.tables_valid = false;
+    D.state = nullptr;  // its tensor maps
     double r_plus = 0.0, r_minus = 0.0;
     fill_grid(*p, h_x, h_r, h_th, h_tx, &r_plus, &r_minus);
     fill_tables(*p, dx, h_r, h_th, h_col, h_row);
@@ -164,10 +176,13 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
     D.dt = p->dt;
     D.tables_valid = true;
   }
-  // The flag must start at zero on every call.
-  if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) {
-    cudaStreamSynchronize(st);
-    return fail(BHR_CUDA_ERROR, "bhr_step_noalloc: clearing the error flag failed");
+  // The flag must start at zero on every call (only a failed call sets it).
+  if (!D.flag_clear) {
+    if (cudaMemsetAsync(flag, 0, sizeof(int), st) != cudaSuccess) {
+      cudaStreamSynchronize(st);
+      return fail(BHR_CUDA_ERROR, "bhr_step_noalloc: clearing the error flag failed");
+    }
+    D.flag_clear = true;
   }
 
   const double third = 0.33333333333333333;
@@ -192,12 +207,59 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
   A.cko = 0.1 * 0.0625 * (1.0 / p->dt);
   A.a2 = p->a * p->a;
   A.m4a = -4.0 * p->a;
+  const char *failed = nullptr;
+  if (resident) {
+    ResidentArgs R{};
+    R.u = state;
+    R.coltab = coltab;
+    R.rowtab = rowtab;
+    R.bb = ctab;
+    R.inbox = reinterpret_cast<ulonglong2 *>(u1);
+    R.err = flag;
+    R.hist = nullptr;
+    R.N = N;
+    R.M = M;
+    R.even_m = A.even_m;
+    R.strips = geom.strips;
+    R.segs = geom.segs;
+    R.rmax = geom.rmax;
+    R.ext[0] = R.ext[1] = -1;
+    R.dt = A.dt;
+    R.cx = A.cx;
+    R.cy = A.cy;
+    R.cyy = A.cyy;
+    R.cko = A.cko;
+    R.a2 = A.a2;
+    R.m4a = A.m4a;
+    if (!D.inbox_valid) {
+      if (cudaMemsetAsync(u1, 0, 2 * kStageDoubles * sizeof(double), st) != cudaSuccess)
+        failed = "clearing the edge words failed";
+      D.inbox_valid = !failed;
+    }
+    for (int k = 0; k < nsteps && !failed && resident; k += R.steps) {
+      R.steps = nsteps - k < kNoAllocLaunchSteps ? nsteps - k : kNoAllocLaunchSteps;
+      R.seq = D.seq;
+      R.close = k + R.steps == nsteps;
+      const cudaError_t e = launch_resident(R, st);
+      if (e == cudaErrorCooperativeLaunchTooLarge && k == 0) {
+        cudaGetLastError();
+        resident = false;  // not enough SMs for one tile each: by stage
+      } else if (e != cudaSuccess) {
+        failed = "resident launch failed";
+      }
+      if (resident) D.seq += 3 * static_cast<unsigned long long>(R.steps);
+    }
+  }
+  if (!resident) {
+    if (D.state != state)
+      if (int rc = encode()) return rc;
+    D.inbox_valid = false;  // u1 and u2 hold stages from here on
+  }
   // The stage kernels request the coefficient tiles before their grid-
   // dependency wait, so the first one of the call is launched without
   // programmatic serialisation: it starts after the table build and the
   // flag reset have completed.  The later ones overlap as in the solver.
-  const char *failed = nullptr;
-  for (int k = 0; k < nsteps && !failed; k++) {
+  for (int k = 0; k < nsteps && !failed && !resident; k++) {
     A.vin = state; A.un = state; A.out = u1;
     if (launch_stage(1, D.maps[0], A, st, /*pdl=*/k > 0) != cudaSuccess) { failed = "stage 1 launch failed"; break; }
     A.vin = u1; A.un = state; A.out = u2;
@@ -205,7 +267,7 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
     A.vin = u2; A.un = state; A.out = state;
     if (launch_stage(3, D.maps[2], A, st) != cudaSuccess) { failed = "stage 3 launch failed"; break; }
   }
-  if (!failed && launch_closure(state, N, M, A.even_m, st) != cudaSuccess) failed = "closure launch failed";
+  if (!failed && (!resident || nsteps == 0) && launch_closure(state, N, M, A.even_m, st) != cudaSuccess) failed = "closure launch failed";
   if (failed) {
     // Let what was launched finish before the lock is released: a later
     // call may rewrite the tables these kernels read.
@@ -218,8 +280,11 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
   const cudaError_t e2 = cudaStreamSynchronize(st);
   if (e1 != cudaSuccess || e2 != cudaSuccess) {
     D.tables_valid = false;
+    D.inbox_valid = false;
+    D.flag_clear = false;
     return fail(BHR_CUDA_ERROR, "bhr_step_noalloc: stream failed");
   }
+  if (h_flag != 0) D.flag_clear = false;
   if (h_flag == BHR_TIMEOUT) return fail(BHR_TIMEOUT, "bhr_step_noalloc: a bounded device wait gave up");
   return BHR_OK;
 }

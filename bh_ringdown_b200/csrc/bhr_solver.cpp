@@ -100,7 +100,7 @@ void free_all(bhr_solver *s) {
   }
   void *ptrs[] = {s->u0,    s->u1,   s->u2,     s->u3,     s->coltab, s->rowtab, s->ctab,   s->rc,     s->th,
                   s->src,   s->ext,  s->integ,  s->wproj,  s->wdedt,  s->rows,   s->recs,   s->rs,  s->psirows,
-                  s->d1f,   s->e2f,  s->colf32, s->rowf32, s->bbf};
+                  s->d1f,   s->e2f,  s->colf32, s->rowf32, s->bbf,    s->inbox,  s->hist,  s->snap,   s->snap_count};
   for (void *q : ptrs)
     if (q) cudaFreeAsync(q, s->stream);
   if (s->g1) cudaGraphExecDestroy(s->g1);
@@ -371,6 +371,31 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
       return BHR_CUDA_ERROR;
     }
   }
+  // A small grid's source-free FP64 SSP-RK3 steps run several to a launch
+  // (not the batch engine's solves, whose tile height the caller fixes, nor
+  // solves whose tiling the environment fixes).
+  if (tile_rows == 0 && p.precision == BHR_FP64 && p.integrator == BHR_SSPRK3) {
+    const char *v = std::getenv("BHR_STAGE_TILING");
+    s->rgeom = resident_geometry(p.N, p.M);
+    if (s->rgeom.ok && (!v || !std::strcmp(v, "resident"))) {
+      const size_t words = resident_inbox_bytes(s->rgeom) / sizeof(ulonglong2);
+      if ((st = dalloc(s, &s->inbox, words)) ||
+          (st = dalloc(s, &s->hist, static_cast<size_t>(4 * kResidentChunk) * p.M)) ||
+          (st = dalloc(s, &s->snap, static_cast<size_t>(4 * kResidentChunk) * p.M)) ||
+          (st = dalloc(s, &s->snap_count, 2))) {
+        free_all(s);
+        delete s;
+        return st;
+      }
+      if ((e = cudaMemsetAsync(s->inbox, 0, words * sizeof(ulonglong2), s->stream))) {
+        set_error(std::string("upload: ") + cudaGetErrorString(e));
+        free_all(s);
+        delete s;
+        return BHR_CUDA_ERROR;
+      }
+      s->resident = true;
+    }
+  }
   // BHR_STAGE_TILING=block8|block16|persistent|block8n|ring fixes the stage
   // tiling of solves whose tiling is not fixed by the caller.
   if (tile_rows == 0) {
@@ -474,9 +499,11 @@ int bhr_solver_info(const bhr_solver *s, bhr_info *info) {
   info->r_plus = s->g.r_plus;
   info->device_bytes = s->bytes;
   info->tile_rows = s->tile_rows;
-  info->persistent = s->persist || s->ring;
-  info->prefetch_ahead = (s->persist || s->ring) ? 0 : stage_prefetch_ahead(s->ahead);
-  info->tiling = s->strip12 ? BHR_TILING_STRIP12
+  const bool resident = s->resident && !s->has_source;
+  info->persistent = s->persist || s->ring || resident;
+  info->prefetch_ahead = (s->persist || s->ring || resident) ? 0 : stage_prefetch_ahead(s->ahead);
+  info->tiling = resident ? BHR_TILING_RESIDENT
+                 : s->strip12 ? BHR_TILING_STRIP12
                  : s->ring ? BHR_TILING_RING
                  : s->narrow ? BHR_TILING_BLOCK8N
                  : s->persist ? BHR_TILING_PERSISTENT
@@ -1144,8 +1171,69 @@ static int capture_steps(bhr_solver *s, int count, cudaGraphExec_t *out) {
   return BHR_OK;
 }
 
+// Steps of a resident solve (source-free): up to kResidentChunk a launch,
+// each followed by the extraction of its steps.  *done: steps enqueued (0 when
+// the device has no room for a cooperative launch: the caller steps by stage).
+static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
+  *done = 0;
+  if (int st = flush_extract(s)) return st;
+  const StageArgs A = solver_stage_args(s);
+  ResidentArgs R{};
+  R.u = s->u0;
+  R.coltab = s->coltab;
+  R.rowtab = s->rowtab;
+  R.bb = s->ctab;
+  R.inbox = s->inbox;
+  R.err = A.err;
+  R.hist = s->hist;
+  R.N = A.N;
+  R.M = A.M;
+  R.even_m = A.even_m;
+  R.strips = s->rgeom.strips;
+  R.segs = s->rgeom.segs;
+  R.rmax = s->rgeom.rmax;
+  // the extraction column, or the two interior columns its closure reads
+  const int a = s->ext_col, N = s->p.N;
+  R.ext[0] = a < 3 ? 3 : a >= N - 3 ? N - 4 : a;
+  R.ext[1] = a < 3 ? 4 : a >= N - 3 ? N - 5 : -1;
+  R.dt = A.dt;
+  R.cx = A.cx;
+  R.cy = A.cy;
+  R.cyy = A.cyy;
+  R.cko = A.cko;
+  R.a2 = A.a2;
+  R.m4a = A.m4a;
+  ChunkArgs C{};
+  C.E = solver_extract_args(s);
+  C.hist = s->hist;
+  C.snap = s->snap;
+  C.count = s->snap_count;
+  while (*done < nsteps) {
+    R.steps = C.steps = std::min(kResidentChunk, nsteps - *done);
+    R.seq = s->rseq;
+    const cudaError_t e = launch_resident(R, s->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      cudaGetLastError();
+      s->resident = false;
+      return BHR_OK;
+    }
+    BHR_CUDA_TRY(e);
+    s->rseq += 3 * static_cast<unsigned long long>(R.steps);
+    BHR_CUDA_TRY(launch_chunk_extract(C, s->stream));
+    *done += R.steps;
+    s->steps_done += R.steps;
+  }
+  return BHR_OK;
+}
+
 static int enqueue_steps(bhr_solver *s, int nsteps) {
   if (nsteps <= 0) return BHR_OK;
+  if (s->resident && !s->has_source) {
+    int done = 0;
+    if (int st = enqueue_resident(s, nsteps, &done)) return st;
+    nsteps -= done;
+    if (nsteps <= 0) return BHR_OK;
+  }
   if (!s->g1)
     if (int st = capture_steps(s, 1, &s->g1)) return st;
   if (nsteps >= kGraphBatch && !s->gb)
@@ -1188,9 +1276,10 @@ int bhr_solver_time_steps(bhr_solver *s, int nsteps, double *ms) {
     return BHR_INVALID_ARG;
   }
   if (int st = solver_wait_records(s, s->steps_done + nsteps + 1)) return st;
-  if (!s->g1)
+  const bool graphs = !s->resident || s->has_source;
+  if (graphs && !s->g1)
     if (int st = capture_steps(s, 1, &s->g1)) return st;
-  if (nsteps >= kGraphBatch && !s->gb)
+  if (graphs && nsteps >= kGraphBatch && !s->gb)
     if (int st = capture_steps(s, kGraphBatch, &s->gb)) return st;
   cudaEvent_t e0, e1;
   BHR_CUDA_TRY(cudaEventCreate(&e0));

@@ -48,6 +48,14 @@ struct bhr_solver {
   int ring = 0;        // 1: 8-row tiles through 2-buffer rings, two 256-thread blocks per SM
   int strip12 = 0;     // 1: stages 1 and 2 in one launch over column strips (FP64 SSP-RK3; stage 3 block8n)
   bhr::StripMaps smaps;
+  // Source-free FP64 SSP-RK3 steps of a small grid: several steps per
+  // cooperative launch (bhr_resident.cu) instead of stage launches.
+  bool resident = false;
+  bhr::ResidentGeom rgeom{};
+  ulonglong2 *inbox = nullptr;   // edge words of the blocks
+  double *hist = nullptr, *snap = nullptr;  // a launch's extraction columns and output snapshots
+  int *snap_count = nullptr;
+  unsigned long long rseq = 1;   // number of the next launch's first edge words
   int steps_done = 0;
   // The extraction of the last step launched has not been launched yet: it
   // runs beside the next step's first stages, or before a host read.

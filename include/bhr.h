@@ -57,14 +57,18 @@ typedef enum bhr_init_kind { BHR_INIT_ZERO = 0, BHR_INIT_GAUSSIAN = 1 } bhr_init
  * 128-thread block, four per SM; 64 x 8 tiles walked by two 256-thread
  * blocks per SM; stages 1 and 2 fused in one launch over 128-column strips
  * (the intermediate stage stays in shared memory; FP64 SSP-RK3 solves, stage
- * 3 as block8n). */
+ * 3 as block8n).  Source-free FP64 SSP-RK3 solves whose grid fits one tile of
+ * 64 columns x up to 32 rows per SM run resident (BHR_TILING_RESIDENT) where
+ * the environment does not fix a tiling: up to 64 steps per launch, each
+ * tile in its SM's shared memory. */
 typedef enum bhr_tiling {
   BHR_TILING_BLOCK8 = 0,
   BHR_TILING_BLOCK16 = 1,
   BHR_TILING_PERSISTENT = 2,
   BHR_TILING_BLOCK8N = 3,
   BHR_TILING_RING = 4,
-  BHR_TILING_STRIP12 = 5
+  BHR_TILING_STRIP12 = 5,
+  BHR_TILING_RESIDENT = 6
 } bhr_tiling;
 
 /* Run parameters.  Replaces HighOrder/parm.h:1-13 (N, M, Xmax, Xmin, Fr, T,
