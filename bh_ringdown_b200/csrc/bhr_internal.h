@@ -65,6 +65,10 @@ struct RunState {
   double timer;   // accumulated as timer += dt (HighOrder/body.cu:214)
 };
 
+// Every stage from the first tile to the last, or stages in turn forward and
+// backward.
+enum StageDir { kSameWay = 0, kForward = 1, kBackward = 2 };
+
 struct StageArgs {
   const double *vin;    // stage input planes (also the TMA source)
   const double *un;     // u^n planes (stages 2 and 3)
@@ -84,6 +88,7 @@ struct StageArgs {
   int ahead;            // one-tile-per-block kernels: each block prefetches into L2 the stage
                         // input of the block this many places later in launch order (0: none,
                         // -1: stage_prefetch_ahead's default; launch_stage resolves it)
+  int dir;              // narrow: the order the stage walks the grid's tiles in (StageDir)
   float *dout;          // mixed precision, stage 1: delta1 = dt L(u^n) in FP32, or nullptr
   double *zout;         // RK4 stage 2: z = (y1 + 2 y2 - u^n)/3, or nullptr
   double dt;            // the stage's step in the combination (RK4: dt/2, dt, dt/6)

@@ -534,11 +534,13 @@ __device__ __forceinline__ void stage_tile(const StageMaps &T, const StageArgs &
 }
 
 // Single solve: the block's tile is blockIdx.y * gridDim.x + blockIdx.x in
-// launch order; the tile `n` places later (kind 1; n = A.ahead, 0: none).
-// The last n blocks name instead the next stage's first n tiles (kind 2):
-// their input, this stage's output and u^n, was written long before and has
-// left L2.
-template <int ROWS>
+// launch order, or that far from the end (kBackward); the tile `n` places
+// later (kind 1; n = A.ahead, 0: none).  Where every stage starts at the first
+// tile (kSameWay), the last n blocks name instead the next stage's first n
+// tiles (kind 2): their input, this stage's output and u^n, was written long
+// before and may have left L2.  Where stages turn, the next one starts on the
+// tiles this one ends on.
+template <int ROWS, int DIR>
 struct GridAhead {
   const StageMaps *T;
   int n;
@@ -549,8 +551,9 @@ struct GridAhead {
     if (L >= ntiles) {
       L -= ntiles;
       kind = 2;
-      if (L >= n || L >= ntiles) return 0;
+      if (DIR != kSameWay || L >= n || L >= ntiles) return 0;
     }
+    if (DIR == kBackward) L = ntiles - 1 - L;
     pm = T;
     c0 = (L % gridDim.x) * TC;
     b0 = (L / gridDim.x) * ROWS;
@@ -576,16 +579,22 @@ struct GroupAhead {
 template <int STAGE, int ROWS>
 __global__ void __launch_bounds__(STAGE_THREADS, 2)
     stage_kernel(const __grid_constant__ StageMaps T, const StageArgs A) {
-  stage_tile<STAGE, ROWS, STAGE_THREADS>(T, A, blockIdx.x * TC, blockIdx.y * ROWS, GridAhead<ROWS>{&T, A.ahead});
+  stage_tile<STAGE, ROWS, STAGE_THREADS>(T, A, blockIdx.x * TC, blockIdx.y * ROWS, GridAhead<ROWS, kSameWay>{&T, A.ahead});
 }
 
 // 8-row tiles on 128-thread blocks: four blocks (16 warps) per SM, so four
-// tiles' loads and computations interleave instead of two.
+// tiles' loads and computations interleave instead of two.  The direction is
+// a template argument: the tile's corner taken from a run-time one costs
+// registers the row work needs (4096 x 128 RK4 48.7 -> 50.6 us a step).
 constexpr int kNarrowThreads = 128;
-template <int STAGE>
+template <int STAGE, int DIR>
 __global__ void __launch_bounds__(kNarrowThreads, 4)
     stage_narrow_kernel(const __grid_constant__ StageMaps T, const StageArgs A) {
-  stage_tile<STAGE, 8, kNarrowThreads>(T, A, blockIdx.x * TC, blockIdx.y * 8, GridAhead<8>{&T, A.ahead});
+  if (DIR == kBackward)
+    stage_tile<STAGE, 8, kNarrowThreads>(T, A, (gridDim.x - 1 - blockIdx.x) * TC, (gridDim.y - 1 - blockIdx.y) * 8,
+                                         GridAhead<8, DIR>{&T, A.ahead});
+  else
+    stage_tile<STAGE, 8, kNarrowThreads>(T, A, blockIdx.x * TC, blockIdx.y * 8, GridAhead<8, DIR>{&T, A.ahead});
 }
 
 // Several solves advanced together: block -> (solve, tile), work item
@@ -1507,8 +1516,10 @@ cudaError_t launch_stage(int stage, const StageMaps &maps, const StageArgs &a_in
     constexpr int S = decltype(sc)::value;
     if (a.narrow) {
       const size_t smem = sizeof(StageSmem<8>) + 128;
-      return launch_ex(pdl, stage_narrow_kernel<S>, dim3(a.N / TC, a.M / 8), dim3(32, kNarrowThreads / 32), smem, st,
-                       maps, a);
+      const dim3 grid(a.N / TC, a.M / 8), block(32, kNarrowThreads / 32);
+      if (a.dir == kForward) return launch_ex(pdl, stage_narrow_kernel<S, kForward>, grid, block, smem, st, maps, a);
+      if (a.dir == kBackward) return launch_ex(pdl, stage_narrow_kernel<S, kBackward>, grid, block, smem, st, maps, a);
+      return launch_ex(pdl, stage_narrow_kernel<S, kSameWay>, grid, block, smem, st, maps, a);
     }
     if (a.ring) {
       const int ntiles = (a.N / TC) * (a.M / kRingRows);
@@ -1542,7 +1553,9 @@ cudaError_t prepare_kernels() {
       cudaError_t r;
       if ((r = cudaFuncSetAttribute(stage_kernel<S, 8>, kSmem, s8)) ||
           (r = cudaFuncSetAttribute(stage_kernel<S, 16>, kSmem, s16)) ||
-          (r = cudaFuncSetAttribute(stage_narrow_kernel<S>, kSmem, s8)) ||
+          (r = cudaFuncSetAttribute(stage_narrow_kernel<S, kSameWay>, kSmem, s8)) ||
+          (r = cudaFuncSetAttribute(stage_narrow_kernel<S, kForward>, kSmem, s8)) ||
+          (r = cudaFuncSetAttribute(stage_narrow_kernel<S, kBackward>, kSmem, s8)) ||
           (r = cudaFuncSetAttribute(stage_persistent_kernel<S>, kSmem, sp)) ||
           (r = cudaFuncSetAttribute(stage_ring_kernel<S>, kSmem, sr)))
         return r;

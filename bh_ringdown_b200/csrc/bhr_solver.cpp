@@ -1016,6 +1016,16 @@ ExtractArgs bhr::solver_extract_args(bhr_solver *s) {
   return E;
 }
 
+// Solves whose states take this much and more are walked back and forth.
+// Measured (us per step, same way -> in turn): 8192 x 128 63.0 -> 62.2 (100 MB
+// of states), 16000 x 256 201 -> 197, 16384 x 256 plunge 204 -> 200; below,
+// where L2 holds the states in any order, nothing is gained and the last
+// blocks' prefetch of the next stage's first tiles would be lost.
+static constexpr size_t kTurnBytes = 96u << 20;
+static bool solver_turns(const bhr_solver *s) {
+  return s->narrow && !s->strip12 && (s->rk4 ? 4 : 3) * sizeof(double) * 4 * static_cast<size_t>(s->p.N) * s->p.M >= kTurnBytes;
+}
+
 // One step.  On the side stream, beside stage 1, the particle source of the
 // next step is built (into the patch buffer this step does not read; its
 // record is selected by the stage step clock, which the previous step
@@ -1028,7 +1038,7 @@ ExtractArgs bhr::solver_extract_args(bhr_solver *s) {
 // 0..5 on the main stream (1..4 around the stages, the final stage between
 // 3 and 4), 6..7 around the extraction and 8..9 around the source on the
 // side stream.
-static int launch_step(bhr_solver *s, cudaEvent_t *ev = nullptr) {
+static int launch_step(bhr_solver *s, cudaEvent_t *ev = nullptr, bool flip = false) {
   auto mark = [&](int i) { return ev ? cudaEventRecord(ev[i], s->stream) : cudaSuccess; };
   auto side_mark = [&](int i) { return ev ? cudaEventRecord(ev[i], s->side) : cudaSuccess; };
   BHR_CUDA_TRY(mark(0));
@@ -1053,6 +1063,14 @@ static int launch_step(bhr_solver *s, cudaEvent_t *ev = nullptr) {
   };
   auto join = [&]() { return side ? cudaStreamWaitEvent(s->stream, s->join, 0) : cudaSuccess; };
   StageArgs A = solver_stage_args(s);
+  // Consecutive stages walk the grid in opposite directions where the states
+  // do not stay in L2 (kTurnBytes), so each starts on the tiles the one before
+  // wrote last; flip is set for steps that begin backward.
+  const bool turns = solver_turns(s);
+  A.dir = !turns ? kSameWay : flip ? kBackward : kForward;
+  auto turn = [&] {
+    if (turns) A.dir = A.dir == kForward ? kBackward : kForward;
+  };
   BHR_CUDA_TRY(mark(1));
   A.vin = s->u0; A.un = s->u0; A.out = s->u1;
   if (s->mixed) {
@@ -1078,12 +1096,15 @@ static int launch_step(bhr_solver *s, cudaEvent_t *ev = nullptr) {
     BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
     BHR_CUDA_TRY(mark(2));
     BHR_CUDA_TRY(fork_extract());
+    turn();
     A.vin = s->u1; A.un = s->u0; A.out = s->u2; A.zout = s->u3;
     BHR_CUDA_TRY(launch_stage(4, s->maps[1], A, s->stream));
+    turn();
     A.vin = s->u2; A.un = s->u0; A.out = s->u1; A.zout = nullptr; A.dt = dt;
     BHR_CUDA_TRY(launch_stage(4, s->maps[3], A, s->stream));
     BHR_CUDA_TRY(mark(3));
     BHR_CUDA_TRY(join());
+    turn();
     A.vin = s->u1; A.un = s->u3; A.out = s->u0; A.dt = dt / 6.0;
     BHR_CUDA_TRY(launch_stage(5, s->maps[4], A, s->stream));
   } else if (s->strip12) {
@@ -1101,10 +1122,12 @@ static int launch_step(bhr_solver *s, cudaEvent_t *ev = nullptr) {
     BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
     BHR_CUDA_TRY(mark(2));
     BHR_CUDA_TRY(fork_extract());
+    turn();
     A.vin = s->u1; A.un = s->u0; A.out = s->u2;
     BHR_CUDA_TRY(launch_stage(2, s->maps[1], A, s->stream));
     BHR_CUDA_TRY(mark(3));
     BHR_CUDA_TRY(join());
+    turn();
     A.vin = s->u2; A.un = s->u0; A.out = s->u0;
     BHR_CUDA_TRY(launch_stage(3, s->maps[2], A, s->stream));
   }
@@ -1151,7 +1174,7 @@ static int capture_steps(bhr_solver *s, int count, cudaGraphExec_t *out) {
   s->pending_extract = true;
   BHR_CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   int st = BHR_OK;
-  for (int i = 0; i < count && st == BHR_OK; i++) st = launch_step(s);
+  for (int i = 0; i < count && st == BHR_OK; i++) st = launch_step(s, nullptr, !s->rk4 && (i & 1));
   cudaError_t e = cudaStreamEndCapture(s->stream, &g);
   s->pending_extract = pending;
   if (st != BHR_OK) {
