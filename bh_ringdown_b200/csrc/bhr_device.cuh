@@ -134,6 +134,24 @@ __device__ __forceinline__ double sqrt_nr(double x) {
 // 1/bir = 1/(B0 + B1 sin^2 theta) (HighOrder/kern.cu:132-149).
 __device__ __forceinline__ double inv_bir(double b0, double b1, double s2) { return rcp_nr(fma(b1, s2, b0)); }
 
+// After a final stage has stored columns a0, a0 + 1 of RPT rows from b0 on:
+// psi at the recorded columns among them (read back by the thread that wrote
+// it, outside the row work, whose registers are all in use) to the history.
+template <int RPT>
+__device__ __forceinline__ void record_columns(double *hist, const int (&ext)[2], const RunState *rs, const int step,
+                                               const double *out, const int N, const int M, const int a0,
+                                               const int b0) {
+  if (hist == nullptr) return;
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    if (ext[e] != a0 && ext[e] != a0 + 1) continue;
+    double *h = hist + static_cast<size_t>(4 * ((rs->ks + step) % kHistSteps) + 2 * e) * M;
+    for (int b = max(b0, 3); b < min(b0 + RPT, M - 3); b++)
+      for (int pl = 0; pl < 2; pl++)
+        h[pl * M + b] = out[(static_cast<size_t>(pl) * M + b) * N + ext[e]];
+  }
+}
+
 // Work item t of a launch group: the index of its solve in the group and
 // the tile corner (tiles of `rows` rows).  Every value read comes from the
 // kernel's parameter space and depends on t alone, so all of a block's

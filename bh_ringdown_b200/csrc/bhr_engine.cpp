@@ -226,7 +226,6 @@ int rebuild(bhr_engine *e) {
       fp64.push_back(i);
     }
     ext[i] = solver_extract_args(s);
-    ext[i].set_ks = 1;  // stages and extraction run in sequence here
     if (s->has_source) {
       src.push_back(solver_source_args(s));
       e->max_ptsx = std::max(e->max_ptsx, s->p.PTSX);

@@ -49,14 +49,12 @@ struct StepRec {
   int col0, row0;           // patch origin: ip - PTSX/2, it - PTSY/2
 };
 
-// Device-side run counters, advanced on the device so a captured step graph
-// can be replayed.  Two step clocks: `ks` (steps whose stages are done; it
-// selects the step's source record and patch buffer) is advanced by a
-// one-thread kernel after a solver step's final stage, or by the extraction
-// where stages and extraction run in sequence (batch engine); `k` (steps
-// extracted; the waveform's clock) by the extraction kernel.  A solver runs
-// the extraction of step n beside stage 2 of step n+1, so until it has run
-// k == ks - 1.
+// Device-side run counters, advanced on the device so a captured sequence of
+// steps can be replayed.  `ks` (steps whose stages are done; with a step's
+// place in its sequence it selects the source record, patch buffer and
+// history slot) is advanced after a sequence's last stage, `k` (steps
+// extracted; the waveform's clock) by the extraction, which runs beside the
+// next sequence or after it.
 struct RunState {
   int k;          // steps extracted
   int nrow;       // waveform rows written
@@ -69,13 +67,16 @@ struct RunState {
 // backward.
 enum StageDir { kSameWay = 0, kForward = 1, kBackward = 2 };
 
+// Steps a solve's history holds: those of two sequences.
+constexpr int kHistSteps = 32;
+
 struct StageArgs {
   const double *vin;    // stage input planes (also the TMA source)
   const double *un;     // u^n planes (stages 2 and 3)
   double *out;          // output planes
   const double *coltab; // [CF_COUNT][N]
   const double *rowtab; // [RF_COUNT][M]
-  const double *src;    // source patch buffers [2][2][PTSY][PTSX] (step k: buffer k % 2) or nullptr
+  const double *src;    // source patch buffers [nbuf][2][PTSY][PTSX] (step k: buffer k % nbuf) or nullptr
   const StepRec *recs;  // per-step records or nullptr
   const RunState *rs;
   int *err;
@@ -91,19 +92,25 @@ struct StageArgs {
   int dir;              // narrow: the order the stage walks the grid's tiles in (StageDir)
   float *dout;          // mixed precision, stage 1: delta1 = dt L(u^n) in FP32, or nullptr
   double *zout;         // RK4 stage 2: z = (y1 + 2 y2 - u^n)/3, or nullptr
+  int nbuf;             // source patch buffers
+  int step;             // this step's place in its launch sequence: step k is rs->ks + step
+  double *hist;         // final stage: psi_re, psi_im at columns ext[0], ext[1] of step k to
+                        // [k % kHistSteps][2][2][M], or nullptr
+  int ext[2];           // -1: none
   double dt;            // the stage's step in the combination (RK4: dt/2, dt, dt/6)
   double cx, cy, cyy, cko;
   double a2, m4a;       // a^2 and -4a: B1 = a2 Dt and BI1 = m4a Dt, the products the column table holds
 };
 
 struct SourceArgs {
-  double *src;          // two patch buffers [2][2][PTSY][PTSX]: step k's patch in buffer k % 2
+  double *src;          // patch buffers [nbuf][2][PTSY][PTSX]: step k's patch in buffer k % nbuf
   const StepRec *recs;
   const RunState *rs;
   const double *r_c;    // [N]
   const double *theta;  // [M]
   int N, M, PTSX, PTSY;
-  int lookahead;        // the patch built is for step rs->ks + lookahead (0 or 1)
+  int nbuf;
+  int lookahead;        // the first patch built is for step rs->ks + lookahead
   int nrecs;            // steps with a record; later steps are skipped
   double a, mass, m, wt;
 };
@@ -118,7 +125,6 @@ struct ExtractArgs {
   double *psirows;      // [max_rows][2][M]: psi at the extraction column on each row's step, or nullptr
   RunState *rs;
   int N, M, ext_col, Fr, max_rows, even_m;
-  int set_ks;           // 1: also advance rs->ks (stages and extraction in sequence)
   double dt, out_start, Xmax;
 };
 
@@ -192,14 +198,16 @@ struct ResidentArgs {
   int close;             // 1: also write the closure of the boundary rows and columns
   double dt, cx, cy, cyy, cko, a2, m4a;
 };
-// Extraction of a resident launch's steps: snapshots of the time integrals
-// on output steps [kResidentChunk][4][M]; count: {first row, rows}.
+// Extraction of a sequence of steps: snapshots of the time integrals on
+// output steps [max_steps][4][M]; count: {first row, rows}.  steps > 0: that
+// many, the s-th in history slot s, and rs->ks is set behind them; 0: the
+// steps from rs->k to rs->ks (max_steps at most), step k in slot k % kHistSteps.
 struct ChunkArgs {
   ExtractArgs E;
   double *hist;          // its closure points are filled in
   double *snap;
   int *count;
-  int steps;
+  int steps, max_steps;
 };
 cudaError_t launch_resident(const ResidentArgs &a, cudaStream_t st);
 cudaError_t launch_chunk_extract(const ChunkArgs &a, cudaStream_t st);
@@ -223,6 +231,10 @@ struct MixedArgs {
   double *u_out;        // stage 3: u^{n+1} planes
   int *err;
   int N, M, even_m;
+  int step;             // stage 3: step, rs, hist and ext as in StageArgs
+  const RunState *rs;
+  double *hist;
+  int ext[2];
   float dt, cx, cy, cyy, cko;
 };
 struct MixedBatch {
@@ -260,14 +272,18 @@ cudaError_t encode_state_maps(void *planes, int N, int M, int rows, CUtensorMap 
 // first launch after tables were rewritten, which the stage kernels read
 // before their grid-dependency wait).
 cudaError_t launch_stage(int stage, const StageMaps &maps, const StageArgs &a, cudaStream_t st, bool pdl = true);
-cudaError_t launch_step_clock(RunState *rs, cudaStream_t st);
+// rs->ks += count, after a sequence's last stage.
+cudaError_t launch_step_clock(RunState *rs, int count, cudaStream_t st);
+// The extraction columns of a state to hist (for stage kernels that do not record them).
+cudaError_t launch_record(const StageArgs &a, cudaStream_t st);
 // Per-point coefficient planes [bb | 1/bir | ee] (3 x M x N) from the tables,
 // and the tensor maps over them and over the column table.
 cudaError_t launch_coef_tables(const double *coltab, const double *rowtab, double *ctab, int N, int M,
                                cudaStream_t st);
 cudaError_t encode_coef_maps(double *ctab, const double *coltab, const double *rowtab, int N, int M, int rows,
                              StageMaps *maps);
-cudaError_t launch_source(const SourceArgs &a, cudaStream_t st);
+// The patches of count steps from rs->ks + lookahead on.
+cudaError_t launch_source(const SourceArgs &a, int count, cudaStream_t st);
 // persist = 1 walks the work-list with one block per SM (16-row tiles);
 // err receives BHR_TIMEOUT if a bounded wait gives up.
 // Stage tilings (the values of bhr_tiling): kernels and tile heights.

@@ -1,8 +1,7 @@
 // bhr_kernels.cu -- sm_100a kernels of the FP64 Teukolsky step.
 //
-// The kernels of one time step (the solver runs the source of the next step
-// and the extraction of the previous one on a side stream beside stages 1
-// and 2, and advances the stage step clock after the final stage):
+// The kernels of a time step (beside the stages of a sequence of steps, a
+// solver builds the sources of the next and extracts the one before):
 //   source_patch  the Gaussian-smeared particle source on its PTSX x PTSY patch
 //                 (HighOrder/kern.cu:755-768 reset + 1185-2683 deposit)
 //   stage<1,2,3>  one SSP-RK3 stage each (classical RK4: stages 1, 4, 4, 5,
@@ -16,7 +15,6 @@
 //   extract       psi at the extraction column, its two time integrals, and
 //                 on output steps the swsh projection and dE/dt
 //                 (HighOrder/body.cu:168-212, HighOrder/proj.c:37-75)
-//   step_clock    one thread: the stage step clock of the next step
 //
 // Storage: each state is four planes (q_re, q_im, p_re, p_im) of M x N
 // doubles, idx(b,a) = N*b + a.  Only interior points 3 <= b < M-3,
@@ -52,7 +50,7 @@ struct __align__(128) StageSmem {
   alignas(128) double rf[RF_COUNT][ROWS];    // TMA box {ROWS, RF_COUNT}: row factors of the tile rows
   uint64_t bar;
   int src_c0, src_r0;           // source patch corner of this step
-  int src_buf;                  // source patch buffer of this step (k % 2)
+  int src_buf;                  // source patch buffer of this step (k % nbuf)
   int done;                     // persistent kernels: warps done with this buffer's tile
   int issued;                   // persistent kernels: load phases issued into this buffer
   int abort;                    // persistent kernels (buffer 0): a bounded wait gave up
@@ -110,18 +108,17 @@ __device__ __forceinline__ void tile_issue_setup(StageSmem<ROWS> &S, const Stage
   tma_load_2d(&S.rf[0][0], &T.rowf, b0, 0, &S.bar);
 }
 
-// Thread 0, after the grid dependency (the stage step clock is advanced
-// after the previous step's final stage, or by its extraction): this step's
-// source patch corner and buffer.
+// Thread 0, after the grid dependency (the step clock is advanced after the
+// previous sequence of steps): this step's source patch corner and buffer.
 // A block barrier publishes it to the other warps.
 template <int ROWS>
 __device__ __forceinline__ void tile_note_source(StageSmem<ROWS> &S, const StageArgs &A) {
   if (A.src != nullptr) {
-    const int k = A.rs->ks;
+    const int k = A.rs->ks + A.step;
     const StepRec &rec = A.recs[k];
     S.src_c0 = rec.col0;
     S.src_r0 = rec.row0;
-    S.src_buf = k & 1;
+    S.src_buf = k % A.nbuf;
   }
 }
 
@@ -531,6 +528,8 @@ __device__ __forceinline__ void stage_tile(const StageMaps &T, const StageArgs &
   tile_close<ROWS, THREADS>(S, A, c0, b0, tid);
   __syncthreads();
   tile_compute<STAGE, ROWS, THREADS, false>(S, A, c0, b0, tx, ty);
+  if (STAGE == 3 || STAGE == 5)
+    record_columns<ROWS / (THREADS / 32)>(A.hist, A.ext, A.rs, A.step, A.out, A.N, A.M, c0 + 2 * tx, b0 + ROWS / (THREADS / 32) * ty);
 }
 
 // Single solve: the block's tile is blockIdx.y * gridDim.x + blockIdx.x in
@@ -1005,10 +1004,10 @@ __global__ void __launch_bounds__(kStripThreads, 1)
   grid_dependency_wait();
   launch_dependents();
   if (tid == 0 && A.src != nullptr) {
-    const int k = A.rs->ks;
+    const int k = A.rs->ks + A.step;
     S.src_c0 = A.recs[k].col0;
     S.src_r0 = A.recs[k].row0;
-    S.src_buf = k & 1;
+    S.src_buf = k % A.nbuf;
   }
   __syncthreads();
   const SrcNote note{S.src_c0, S.src_r0, S.src_buf};
@@ -1186,16 +1185,16 @@ __global__ void closure_ends_kernel(double *P, int N, int M) {
 // factors, and the per-point work is the bilinear sum and the epilogue.
 constexpr int kSrcRows = 4;
 
-__device__ __forceinline__ void source_rows(const SourceArgs &A, const int j0, const int k) {
+__device__ __forceinline__ void source_rows(const SourceArgs &A, const int j0, const int k, const int step) {
   __shared__ double rowf[kSrcRows][5];  // T0, T1, T2, cos theta, sin theta
   __shared__ int rok[kSrcRows];
-  // The patch of step k goes to buffer k % 2; a lookahead past the last
-  // record builds nothing.
-  const int kstep = A.rs->ks + A.lookahead;
+  // The patch of step k goes to buffer k % nbuf; none is built past the last
+  // record.
+  const int kstep = A.rs->ks + A.lookahead + step;
   if (kstep >= A.nrecs) return;  // uniform across the block
   // By value: the stores to the patch below must not force reloads.
   const StepRec rec = A.recs[kstep];
-  double *__restrict__ src = A.src + static_cast<size_t>(kstep & 1) * 2 * A.PTSX * A.PTSY;
+  double *__restrict__ src = A.src + static_cast<size_t>(kstep % A.nbuf) * 2 * A.PTSX * A.PTSY;
   const double a = A.a, mass = A.mass;
   if (k < kSrcRows) {
     const int row = j0 + k + rec.row0;
@@ -1264,10 +1263,11 @@ __device__ __forceinline__ void source_rows(const SourceArgs &A, const int j0, c
   }
 }
 
+// blockIdx.y: the step of the sequence.
 __global__ void source_patch_kernel(const SourceArgs A) {
   grid_dependency_wait();
   launch_dependents();
-  source_rows(A, blockIdx.x * kSrcRows, threadIdx.x);
+  source_rows(A, blockIdx.x * kSrcRows, threadIdx.x, blockIdx.y);
 }
 
 // Sourced solves of a batch: blockIdx.y picks the solve.
@@ -1275,7 +1275,7 @@ __global__ void source_batch_kernel(const SourceArgs *args) {
   grid_dependency_wait();
   launch_dependents();
   const SourceArgs &A = args[blockIdx.y];
-  if (static_cast<int>(blockIdx.x) * kSrcRows < A.PTSY) source_rows(A, blockIdx.x * kSrcRows, threadIdx.x);
+  if (static_cast<int>(blockIdx.x) * kSrcRows < A.PTSY) source_rows(A, blockIdx.x * kSrcRows, threadIdx.x, 0);
 }
 
 // ---- extraction, integration, projection (HighOrder/body.cu:168-212) ------
@@ -1283,12 +1283,10 @@ constexpr int kExtractThreads = 256;
 constexpr int kSums = 15;
 
 // Every kernel calls griddepcontrol.wait before it lets its dependents
-// start, and a solver's extraction is ordered after the previous one
-// through the step's stage 3 (which waits for it), so when this kernel
-// starts, the previous step's extraction (the only writer of integ, rows,
-// k, nrow and timer) has completed: those, and the weights written at
-// set-up, are read before the wait; only psi at the extraction column waits
-// for stage 3.
+// start, so when this kernel starts, the previous extraction (the only writer
+// of integ, rows, k, nrow and timer) has completed: those, and the weights
+// written at set-up, are read before the wait; only psi at the extraction
+// column waits for the final stage.
 __device__ __forceinline__ void extract_body(const ExtractArgs &A) {
   __shared__ double red[kExtractThreads / 32][kSums];
   const int tid = threadIdx.x;
@@ -1367,18 +1365,31 @@ __device__ __forceinline__ void extract_body(const ExtractArgs &A) {
     }
     A.rs->timer = timer + A.dt;
     A.rs->k = k + 1;
-    if (A.set_ks) A.rs->ks = k + 1;
+    A.rs->ks = k + 1;
   }
 }
 
 __global__ void __launch_bounds__(kExtractThreads) extract_kernel(const ExtractArgs A) { extract_body(A); }
 
-// After a solver step's final stage: advance the stage step clock.  Its own
-// launch, because every block of the final stage reads the clock.
-__global__ void step_clock_kernel(RunState *rs) {
+// After a sequence's last stage: its own launch, because every block of the
+// stages reads the clock.
+__global__ void step_clock_kernel(RunState *rs, int count) {
   grid_dependency_wait();
   launch_dependents();
-  if (threadIdx.x == 0) rs->ks += 1;
+  if (threadIdx.x == 0) rs->ks += count;
+}
+
+// psi at the recorded columns of a state, for stage kernels that do not
+// record it themselves.
+__global__ void record_kernel(const StageArgs A) {
+  grid_dependency_wait();
+  launch_dependents();
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < 3 || b >= A.M - 3) return;
+  for (int e = 0; e < 2; e++)
+    for (int pl = 0; pl < 2 && A.ext[e] >= 0; pl++)
+      A.hist[static_cast<size_t>(4 * ((A.rs->ks + A.step) % kHistSteps) + 2 * e + pl) * A.M + b] =
+          A.out[(static_cast<size_t>(pl) * A.M + b) * A.N + A.ext[e]];
 }
 
 // One block per solve of a batch.
@@ -1648,12 +1659,18 @@ cudaError_t launch_extract_batch(const ExtractArgs *args, int nsolves, cudaStrea
   return launch_pdl(extract_batch_kernel, dim3(nsolves), dim3(kExtractThreads), 0, st, args);
 }
 
-cudaError_t launch_source(const SourceArgs &a, cudaStream_t st) {
-  return launch_pdl(source_patch_kernel, dim3((a.PTSY + kSrcRows - 1) / kSrcRows), dim3(std::max(a.PTSX, kSrcRows)), 0,
-                    st, a);
+cudaError_t launch_source(const SourceArgs &a, int count, cudaStream_t st) {
+  return launch_pdl(source_patch_kernel, dim3((a.PTSY + kSrcRows - 1) / kSrcRows, count),
+                    dim3(std::max(a.PTSX, kSrcRows)), 0, st, a);
 }
 
-cudaError_t launch_step_clock(RunState *rs, cudaStream_t st) { return launch_pdl(step_clock_kernel, dim3(1), dim3(32), 0, st, rs); }
+cudaError_t launch_step_clock(RunState *rs, int count, cudaStream_t st) {
+  return launch_pdl(step_clock_kernel, dim3(1), dim3(32), 0, st, rs, count);
+}
+
+cudaError_t launch_record(const StageArgs &a, cudaStream_t st) {
+  return launch_pdl(record_kernel, dim3((a.M + 127) / 128), dim3(128), 0, st, a);
+}
 
 cudaError_t launch_extract(const ExtractArgs &a, cudaStream_t st) {
   return launch_pdl(extract_kernel, dim3(1), dim3(kExtractThreads), 0, st, a);

@@ -330,6 +330,7 @@ __device__ __forceinline__ void mixed_tile(const MixedMaps &T, const MixedArgs &
   };
   if (!lo_cols && !hi_cols) rows(std::true_type{});
   else rows(std::false_type{});
+  if (STAGE == 3) record_columns<RPT>(A.hist, A.ext, A.rs, A.step, A.u_out, N, M, a0, b0 + RPT * ty);
 }
 
 template <int STAGE>

@@ -559,20 +559,22 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_integrate_kernel(const __
   launch_dependents();
   const ExtractArgs &E = A.E;
   const int M = E.M, tid = threadIdx.x, k0 = E.rs->k, row0 = E.rs->nrow, phase0 = k0 % E.Fr;
+  const int steps = A.steps > 0 ? A.steps : min(E.rs->ks - k0, A.max_steps);
+  auto slot = [&](const int s) { return A.hist + static_cast<size_t>(4 * (A.steps > 0 ? s : (k0 + s) % kHistSteps)) * M; };
   const int a = E.ext_col, N = E.N;
   const bool end_col = a < 3 || a >= N - 3;
-  for (int i = tid; i < A.steps * (end_col ? 4 : 2) * 2; i += kChunkThreads) {
+  for (int i = tid; i < steps * (end_col ? 4 : 2) * 2; i += kChunkThreads) {
     const int hi = i & 1, k = i >> 1;
-    double *h = A.hist + static_cast<size_t>(end_col ? k : 4 * (k >> 1) + (k & 1)) * M;  // (step, column, plane)
+    double *h = end_col ? slot(k >> 2) + (k & 3) * M : slot(k >> 1) + (k & 1) * M;  // (step, column, plane)
     const double f1 = hi ? h[M - 4] : h[3], f2 = hi ? h[M - 5] : h[4];
 #pragma unroll
     for (int d = 1; d <= 3; d++) h[hi ? M - 4 + d : 3 - d] = E.even_m ? extrap(f1, f2, d) : 0.0;
   }
   __syncthreads();
   if (end_col) {
-    for (int i = tid; i < A.steps * 2 * M; i += kChunkThreads) {
+    for (int i = tid; i < steps * 2 * M; i += kChunkThreads) {
       const int k = i / M;
-      double *h = A.hist + static_cast<size_t>(4 * (k >> 1) + (k & 1)) * M + (i - k * M);
+      double *h = slot(k >> 1) + (k & 1) * M + (i - k * M);
       h[0] = extrap(h[0], h[2 * M], a < 3 ? 3 - a : a - (N - 4));
     }
     __syncthreads();
@@ -582,16 +584,16 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_integrate_kernel(const __
     double ir = E.integ[b], ii = E.integ[M + b], dr = E.integ[2 * M + b], di = E.integ[3 * M + b];
     double pr[kBatch], pi[kBatch];
     int n = 0, phase = phase0;  // phase: k mod Fr
-    for (int s0 = 0; s0 < A.steps; s0 += kBatch) {
+    for (int s0 = 0; s0 < steps; s0 += kBatch) {
 #pragma unroll
       for (int s = 0; s < kBatch; s++) {
-        const double *h = A.hist + static_cast<size_t>(4 * min(s0 + s, A.steps - 1)) * M + b;
+        const double *h = slot(min(s0 + s, steps - 1)) + b;
         pr[s] = h[0];
         pi[s] = h[M];
       }
 #pragma unroll
       for (int s = 0; s < kBatch; s++) {
-        if (s0 + s >= A.steps) break;
+        if (s0 + s >= steps) break;
         if (!isfinite(pr[s]) || !isfinite(pi[s])) bad = 1;
         ir = ir + pr[s] * E.dt;
         ii = ii + pi[s] * E.dt;
@@ -612,7 +614,7 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_integrate_kernel(const __
           n++;
         }
         if (++phase == E.Fr) phase = 0;
-        if (s0 + s + 1 == A.steps) {
+        if (s0 + s + 1 == steps) {
           E.ext[b] = pr[s];
           E.ext[M + b] = pi[s];
         }
@@ -627,7 +629,7 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_integrate_kernel(const __
   if (tid == 0) {
     double t = E.rs->timer;
     int n = 0, phase = phase0;
-    for (int s = 0; s < A.steps; s++) {
+    for (int s = 0; s < steps; s++) {
       if (phase == 0 && static_cast<double>(k0 + s) * E.dt >= E.out_start && row0 + n < E.max_rows)
         E.rows[static_cast<size_t>(row0 + n++) * 16] = t - E.Xmax;
       if (++phase == E.Fr) phase = 0;
@@ -637,8 +639,8 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_integrate_kernel(const __
     A.count[1] = n;
     E.rs->timer = t;
     E.rs->nrow = row0 + n;
-    E.rs->k = k0 + A.steps;
-    E.rs->ks = k0 + A.steps;
+    E.rs->k = k0 + steps;
+    if (A.steps > 0) E.rs->ks = k0 + steps;
   }
 }
 
@@ -757,7 +759,7 @@ cudaError_t launch_resident(const ResidentArgs &a, cudaStream_t st) {
 cudaError_t launch_chunk_extract(const ChunkArgs &a, cudaStream_t st) {
   cudaError_t e = launch_pdl(chunk_integrate_kernel, dim3(1), dim3(kChunkThreads), 0, st, a);
   if (e != cudaSuccess) return e;
-  return launch_pdl(chunk_project_kernel, dim3(a.steps / a.E.Fr + 1), dim3(kChunkThreads), 0, st, a);
+  return launch_pdl(chunk_project_kernel, dim3(a.max_steps / a.E.Fr + 1), dim3(kChunkThreads), 0, st, a);
 }
 
 }  // namespace bhr

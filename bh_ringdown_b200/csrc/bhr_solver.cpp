@@ -4,7 +4,8 @@
 // all state is per solve (no __device__ globals), the trajectory is read
 // once into memory and turned into per-step source records before the
 // loop, the extraction integrals and the projection stay on the device, and
-// a step is five kernel launches on one stream with no host round trip.
+// steps run in sequences of stage launches on one stream with no host round
+// trip.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -42,7 +43,20 @@ void set_error(const std::string &msg) { g_err = msg; }
 
 using namespace bhr;
 
-static constexpr int kGraphBatch = 16;
+// Steps launched as one sequence.
+static constexpr int kSequence = 16;
+static_assert(2 * kSequence <= kHistSteps, "the history holds two sequences");
+// A sequence is captured into a graph when at least kGraphSteps are left to
+// run, or the grid has fewer than kDirectPoints points.  A graph of 16 steps
+// costs 3.5 ms to capture, instantiate and destroy (4096 x 128 RK4, 600 steps:
+// 10 % of the solve) and frees the host of long runs; launched directly, a
+// step costs the host 10-15 us, which steps of small grids do not hide (us a
+// step, graph and direct: 2048 x 128 mixed 22.2 and 24.1, 1024 x 64 sourced 11.7
+// and 14.8, 4096 x 128 sourced 35.8 and 35.3).
+static constexpr int kGraphSteps = 4096;
+static constexpr size_t kDirectPoints = 400000;
+// Patch buffers of a solve take at most this much (two at least).
+static constexpr size_t kPatchBytes = 64u << 20;
 
 namespace {
 
@@ -116,9 +130,8 @@ void free_all(bhr_solver *s) {
   }
   if (s->fork) cudaEventDestroy(s->fork);
   if (s->join) cudaEventDestroy(s->join);
-  if (s->fork2) cudaEventDestroy(s->fork2);
   s->stream = s->side = nullptr;
-  s->fork = s->join = s->fork2 = nullptr;
+  s->fork = s->join = nullptr;
 }
 
 // The device's default memory pool keeps freed blocks for reuse instead of
@@ -147,8 +160,7 @@ double tortoise(double r, double a, double rpl, double rmn) {
 }  // namespace
 
 static int autotune_rows(bhr_solver *s);
-static int flush_extract(bhr_solver *s);
-
+static cudaError_t launch_first_sources(bhr_solver *s);
 
 extern "C" {
 
@@ -300,17 +312,20 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
 
   const size_t NM = static_cast<size_t>(p.N) * p.M;
   int st = BHR_OK;
-  // The side stream (source, extraction: a few blocks beside the stages)
+  // Patch buffers: this sequence's and the next one's steps, two at least.
+  const size_t patch = 2 * static_cast<size_t>(p.PTSX) * p.PTSY;
+  const bool engine = tile_rows != 0;  // which steps its solves one by one
+  s->nbuf = engine ? 2 : 2 * static_cast<int>(std::max<size_t>(1, std::min<size_t>(kSequence, kPatchBytes / (16 * patch))));
+  // The side stream (sources, extraction: a few blocks beside the stages)
   // gets the device's highest priority, so its blocks take the first SM
   // slots that free up.
   int hi_prio = 0;
   if (cudaSetDevice(p.device) != cudaSuccess || prepare_kernels() != cudaSuccess || keep_pool_memory(p.device) ||
       cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaDeviceGetStreamPriorityRange(nullptr, &hi_prio) != cudaSuccess ||
-      cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, hi_prio) != cudaSuccess ||
-      cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&s->fork2, cudaEventDisableTiming) != cudaSuccess) {
+      (!engine && (cudaDeviceGetStreamPriorityRange(nullptr, &hi_prio) != cudaSuccess ||
+                   cudaStreamCreateWithPriority(&s->side, cudaStreamNonBlocking, hi_prio) != cudaSuccess ||
+                   cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) != cudaSuccess ||
+                   cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming) != cudaSuccess))) {
     set_error("cannot set device / create stream");
     delete s;
     return BHR_CUDA_ERROR;
@@ -319,7 +334,7 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
       (st = dalloc(s, &s->coltab, static_cast<size_t>(CF_COUNT) * p.N)) ||
       (st = dalloc(s, &s->rowtab, static_cast<size_t>(RF_COUNT) * p.M)) || (st = dalloc(s, &s->ctab, NM)) ||
       (st = dalloc(s, &s->rc, p.N)) ||
-      (st = dalloc(s, &s->th, p.M)) || (st = dalloc(s, &s->src, 4 * static_cast<size_t>(p.PTSX) * p.PTSY)) ||
+      (st = dalloc(s, &s->th, p.M)) || (st = dalloc(s, &s->src, s->nbuf * patch)) ||
       (st = dalloc(s, &s->ext, 2 * static_cast<size_t>(p.M))) || (st = dalloc(s, &s->integ, 4 * static_cast<size_t>(p.M))) ||
       (st = dalloc(s, &s->wproj, 7 * static_cast<size_t>(p.M))) || (st = dalloc(s, &s->wdedt, p.M)) ||
       (st = dalloc(s, &s->rows, 16 * static_cast<size_t>(s->max_rows))) ||
@@ -350,7 +365,7 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
       (e = launch_coef_tables(s->coltab, s->rowtab, s->ctab, p.N, p.M, s->stream)) ||
       (e = cudaMemsetAsync(s->u1, 0, 4 * NM * 8, s->stream)) || (e = cudaMemsetAsync(s->u2, 0, 4 * NM * 8, s->stream)) ||
       (e = cudaMemsetAsync(s->integ, 0, 4 * p.M * 8, s->stream)) || (e = cudaMemsetAsync(s->ext, 0, 2 * p.M * 8, s->stream)) ||
-      (e = cudaMemsetAsync(s->src, 0, 4 * static_cast<size_t>(p.PTSX) * p.PTSY * 8, s->stream)) ||
+      (e = cudaMemsetAsync(s->src, 0, s->nbuf * patch * 8, s->stream)) ||
       (e = cudaMemsetAsync(s->rs, 0, sizeof(RunState), s->stream)) || (e = cudaStreamSynchronize(s->stream))) {
     set_error(std::string("upload: ") + cudaGetErrorString(e));
     if (dfac) cudaFreeAsync(dfac, s->stream);
@@ -379,10 +394,7 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
     s->rgeom = resident_geometry(p.N, p.M);
     if (s->rgeom.ok && (!v || !std::strcmp(v, "resident"))) {
       const size_t words = resident_inbox_bytes(s->rgeom) / sizeof(ulonglong2);
-      if ((st = dalloc(s, &s->inbox, words)) ||
-          (st = dalloc(s, &s->hist, static_cast<size_t>(4 * kResidentChunk) * p.M)) ||
-          (st = dalloc(s, &s->snap, static_cast<size_t>(4 * kResidentChunk) * p.M)) ||
-          (st = dalloc(s, &s->snap_count, 2))) {
+      if ((st = dalloc(s, &s->inbox, words))) {
         free_all(s);
         delete s;
         return st;
@@ -394,6 +406,14 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
         return BHR_CUDA_ERROR;
       }
       s->resident = true;
+    }
+  }
+  if (tile_rows == 0) {
+    const size_t n = static_cast<size_t>(4 * (s->resident ? std::max(kResidentChunk, kHistSteps) : kHistSteps)) * p.M;
+    if ((st = dalloc(s, &s->hist, n)) || (st = dalloc(s, &s->snap, n)) || (st = dalloc(s, &s->snap_count, 2))) {
+      free_all(s);
+      delete s;
+      return st;
     }
   }
   // BHR_STAGE_TILING=block8|block16|persistent|block8n|ring fixes the stage
@@ -489,8 +509,6 @@ int bhr_solver_info(const bhr_solver *s, bhr_info *info) {
   info->nt = s->nt;
   info->Fr = s->Fr;
   info->steps_done = s->steps_done;
-  // Reading the row count completes the last step's extraction first.
-  if (int st = flush_extract(const_cast<bhr_solver *>(s))) return st;
   RunState rs{};
   BHR_CUDA_TRY(cudaMemcpyAsync(&rs, s->rs, sizeof(rs), cudaMemcpyDeviceToHost, s->stream));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -680,8 +698,9 @@ static void stop_records(bhr_solver *s) {
   s->rec_stop = false;
 }
 
-int bhr::solver_wait_records(bhr_solver *s, int upto) {
+int bhr::solver_wait_records(bhr_solver *s, int upto, int ahead) {
   if (!s->has_source) return BHR_OK;
+  const int more = static_cast<int>(std::min<long long>(static_cast<long long>(upto) + ahead, s->nt));
   upto = std::min(upto, s->nt);
   std::unique_lock<std::mutex> lock(s->rec_mu);
   if (s->rec_unusable) {
@@ -701,6 +720,7 @@ int bhr::solver_wait_records(bhr_solver *s, int upto) {
     set_error("trajectory records end at step " + std::to_string(s->rec_ready));
     return BHR_INVALID_ARG;
   }
+  if (s->rec_ready < more) s->rec_cv.wait(lock, [&] { return s->rec_ready >= more || s->rec_bad >= 0 || !s->rec_running; });
   return BHR_OK;
 }
 
@@ -715,7 +735,6 @@ int bhr_solver_set_trajectory(bhr_solver *s, const double *rows, int nrows) {
     return BHR_INVALID_ARG;
   }
   cudaSetDevice(s->p.device);
-  if (int st = flush_extract(s)) return st;
   stop_records(s);
   {
     // Until this call succeeds the solve has no usable records: a sourced
@@ -778,8 +797,8 @@ int bhr_solver_set_trajectory(bhr_solver *s, const double *rows, int nrows) {
       return BHR_OUT_OF_MEMORY;
     }
   }
-  // The patch of the current step (later patches are built one step ahead).
-  BHR_CUDA_TRY(launch_source(solver_source_args(s), s->stream));
+  // The patches of the first sequence (later ones are built beside the stages).
+  BHR_CUDA_TRY(launch_first_sources(s));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
   // The launch arguments now carry the source and the new records: step
   // graphs captured before (steps taken without a trajectory) are rebuilt.
@@ -936,6 +955,8 @@ StageArgs bhr::solver_stage_args(bhr_solver *s) {
   A.src = s->has_source ? s->src : nullptr;
   A.recs = s->recs;
   A.rs = s->rs;
+  A.nbuf = s->nbuf;
+  A.ext[0] = A.ext[1] = -1;
   A.err = &s->rs->err;
   A.N = p.N;
   A.M = p.M;
@@ -964,6 +985,8 @@ MixedArgs bhr::solver_mixed_args(bhr_solver *s) {
   X.N = A.N;
   X.M = A.M;
   X.even_m = A.even_m;
+  X.rs = A.rs;
+  X.ext[0] = X.ext[1] = -1;
   X.dt = static_cast<float>(A.dt);
   X.cx = static_cast<float>(A.cx);
   X.cy = static_cast<float>(A.cy);
@@ -984,6 +1007,7 @@ SourceArgs bhr::solver_source_args(bhr_solver *s) {
   S.M = p.M;
   S.PTSX = p.PTSX;
   S.PTSY = p.PTSY;
+  S.nbuf = s->nbuf;
   S.lookahead = 0;
   S.nrecs = s->nt;
   S.a = p.a;
@@ -1026,66 +1050,58 @@ static bool solver_turns(const bhr_solver *s) {
   return s->narrow && !s->strip12 && (s->rk4 ? 4 : 3) * sizeof(double) * 4 * static_cast<size_t>(s->p.N) * s->p.M >= kTurnBytes;
 }
 
-// One step.  On the side stream, beside stage 1, the particle source of the
-// next step is built (into the patch buffer this step does not read; its
-// record is selected by the stage step clock, which the previous step
-// advanced), and beside stage 2 (RK4: stages 2-3) the previous step's
-// extraction runs when it is pending: it reads only u^n, which the stages
-// before the last only read, and its own accumulators.  The side branch
-// joins before the final stage, which overwrites u^n; a one-thread kernel
-// then advances the stage step clock.  This step's extraction is left
-// pending (flush_extract launches it, or the next step).  `ev` (10 events):
-// 0..5 on the main stream (1..4 around the stages, the final stage between
-// 3 and 4), 6..7 around the extraction and 8..9 around the source on the
-// side stream.
-static int launch_step(bhr_solver *s, cudaEvent_t *ev = nullptr, bool flip = false) {
+// The columns a step's history keeps: the extraction column, or the two
+// interior ones its closure is made of.
+static void history_columns(const bhr_solver *s, int ext[2]) {
+  const int a = s->ext_col, N = s->p.N;
+  ext[0] = a < 3 ? 3 : a >= N - 3 ? N - 4 : a;
+  ext[1] = a < 3 ? 4 : a >= N - 3 ? N - 5 : -1;
+}
+
+// The stages of one step, the `step`-th of its sequence.  record: psi at the
+// history columns goes to the history.  flip: the step begins backward, where
+// stages turn.  `ev`: 4 events around the stages (the final one, and RK4's
+// third, between the last two).
+static int launch_stages(bhr_solver *s, int step, bool record, bool flip, cudaEvent_t *ev = nullptr) {
   auto mark = [&](int i) { return ev ? cudaEventRecord(ev[i], s->stream) : cudaSuccess; };
-  auto side_mark = [&](int i) { return ev ? cudaEventRecord(ev[i], s->side) : cudaSuccess; };
-  BHR_CUDA_TRY(mark(0));
-  if (s->has_source) {
-    BHR_CUDA_TRY(cudaEventRecord(s->fork, s->stream));
-    BHR_CUDA_TRY(cudaStreamWaitEvent(s->side, s->fork, 0));
-    SourceArgs S = solver_source_args(s);
-    S.lookahead = 1;
-    BHR_CUDA_TRY(side_mark(8));
-    BHR_CUDA_TRY(launch_source(S, s->side));
-    BHR_CUDA_TRY(side_mark(9));
-  }
-  const bool extract = s->pending_extract;
-  const bool side = extract || s->has_source;
-  auto fork_extract = [&]() -> cudaError_t {
-    if (!extract) return side ? cudaEventRecord(s->join, s->side) : cudaSuccess;
-    cudaError_t e;
-    if ((e = cudaEventRecord(s->fork2, s->stream)) || (e = cudaStreamWaitEvent(s->side, s->fork2, 0)) ||
-        (e = side_mark(6)) || (e = launch_extract(solver_extract_args(s), s->side)) || (e = side_mark(7)))
-      return e;
-    return cudaEventRecord(s->join, s->side);
-  };
-  auto join = [&]() { return side ? cudaStreamWaitEvent(s->stream, s->join, 0) : cudaSuccess; };
   StageArgs A = solver_stage_args(s);
+  A.step = step;
   // Consecutive stages walk the grid in opposite directions where the states
   // do not stay in L2 (kTurnBytes), so each starts on the tiles the one before
-  // wrote last; flip is set for steps that begin backward.
+  // wrote last.
   const bool turns = solver_turns(s);
   A.dir = !turns ? kSameWay : flip ? kBackward : kForward;
   auto turn = [&] {
     if (turns) A.dir = A.dir == kForward ? kBackward : kForward;
   };
-  BHR_CUDA_TRY(mark(1));
+  auto final_stage = [&](int stage, int map) -> cudaError_t {
+    if (!record) return launch_stage(stage, s->maps[map], A, s->stream);
+    A.hist = s->hist;
+    history_columns(s, A.ext);
+    if (!s->persist && !s->ring) return launch_stage(stage, s->maps[map], A, s->stream);
+    const StageArgs R = A;  // the kernels that walk several tiles do not record
+    A.hist = nullptr;
+    const cudaError_t e = launch_stage(stage, s->maps[map], A, s->stream);
+    return e != cudaSuccess ? e : launch_record(R, s->stream);
+  };
+  BHR_CUDA_TRY(mark(0));
   A.vin = s->u0; A.un = s->u0; A.out = s->u1;
   if (s->mixed) {
     // u1 in FP64 and delta1 in FP32, then the FP32 stages 2 and 3.
     A.dout = s->d1f;
     BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
-    BHR_CUDA_TRY(mark(2));
-    BHR_CUDA_TRY(fork_extract());
+    BHR_CUDA_TRY(mark(1));
     MixedArgs X = solver_mixed_args(s);
     X.e_out = s->e2f;
     BHR_CUDA_TRY(launch_mixed_stage(2, s->mmaps[0], X, s->stream));
-    BHR_CUDA_TRY(mark(3));
-    BHR_CUDA_TRY(join());
+    BHR_CUDA_TRY(mark(2));
     X.e_out = nullptr;
     X.u_out = s->u0;
+    X.step = step;
+    if (record) {
+      X.hist = s->hist;
+      history_columns(s, X.ext);
+    }
     BHR_CUDA_TRY(launch_mixed_stage(3, s->mmaps[1], X, s->stream));
   } else if (s->rk4) {
     // Classical RK4, the step's source held fixed in all four stages:
@@ -1094,56 +1110,83 @@ static int launch_step(bhr_solver *s, cudaEvent_t *ev = nullptr, bool flip = fal
     const double dt = A.dt;
     A.dt = 0.5 * dt;
     BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
-    BHR_CUDA_TRY(mark(2));
-    BHR_CUDA_TRY(fork_extract());
+    BHR_CUDA_TRY(mark(1));
     turn();
     A.vin = s->u1; A.un = s->u0; A.out = s->u2; A.zout = s->u3;
     BHR_CUDA_TRY(launch_stage(4, s->maps[1], A, s->stream));
     turn();
     A.vin = s->u2; A.un = s->u0; A.out = s->u1; A.zout = nullptr; A.dt = dt;
     BHR_CUDA_TRY(launch_stage(4, s->maps[3], A, s->stream));
-    BHR_CUDA_TRY(mark(3));
-    BHR_CUDA_TRY(join());
+    BHR_CUDA_TRY(mark(2));
     turn();
     A.vin = s->u1; A.un = s->u3; A.out = s->u0; A.dt = dt / 6.0;
-    BHR_CUDA_TRY(launch_stage(5, s->maps[4], A, s->stream));
-  } else if (s->strip12) {
-    // Stages 1 and 2 in one launch (u1 stays on chip), beside the previous
-    // step's extraction, which reads only u^n.
-    BHR_CUDA_TRY(fork_extract());
-    A.vin = s->u0; A.un = s->u0; A.out = s->u2;
-    BHR_CUDA_TRY(launch_stage12_strip(s->smaps, A, s->stream));
-    BHR_CUDA_TRY(mark(2));
-    BHR_CUDA_TRY(mark(3));
-    BHR_CUDA_TRY(join());
-    A.vin = s->u2; A.un = s->u0; A.out = s->u0;
-    BHR_CUDA_TRY(launch_stage(3, s->maps[2], A, s->stream));
+    BHR_CUDA_TRY(final_stage(5, 4));
   } else {
-    BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
+    if (s->strip12) {  // stages 1 and 2 in one launch (u1 stays on chip)
+      A.out = s->u2;
+      BHR_CUDA_TRY(launch_stage12_strip(s->smaps, A, s->stream));
+      BHR_CUDA_TRY(mark(1));
+    } else {
+      BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
+      BHR_CUDA_TRY(mark(1));
+      turn();
+      A.vin = s->u1; A.un = s->u0; A.out = s->u2;
+      BHR_CUDA_TRY(launch_stage(2, s->maps[1], A, s->stream));
+    }
     BHR_CUDA_TRY(mark(2));
-    BHR_CUDA_TRY(fork_extract());
-    turn();
-    A.vin = s->u1; A.un = s->u0; A.out = s->u2;
-    BHR_CUDA_TRY(launch_stage(2, s->maps[1], A, s->stream));
-    BHR_CUDA_TRY(mark(3));
-    BHR_CUDA_TRY(join());
     turn();
     A.vin = s->u2; A.un = s->u0; A.out = s->u0;
-    BHR_CUDA_TRY(launch_stage(3, s->maps[2], A, s->stream));
+    BHR_CUDA_TRY(final_stage(3, 2));
   }
-  BHR_CUDA_TRY(mark(4));
-  BHR_CUDA_TRY(launch_step_clock(s->rs, s->stream));
-  BHR_CUDA_TRY(mark(5));
-  s->pending_extract = true;
+  BHR_CUDA_TRY(mark(3));
   return BHR_OK;
 }
 
-// The last step's extraction, before anything reads the waveform, the
-// extraction buffers or the run counters, or replaces the state.
-static int flush_extract(bhr_solver *s) {
-  if (!s->pending_extract) return BHR_OK;
-  BHR_CUDA_TRY(launch_extract(solver_extract_args(s), s->stream));
-  s->pending_extract = false;
+static int sequence_length(const bhr_solver *s) { return s->has_source ? s->nbuf / 2 : kSequence; }
+
+// The patches of a sequence from the current step on, before the first.
+static cudaError_t launch_first_sources(bhr_solver *s) {
+  return launch_source(solver_source_args(s), s->nbuf / 2, s->stream);
+}
+
+// The extraction of the steps done and not yet extracted (kSequence at most).
+static cudaError_t launch_extraction(bhr_solver *s, cudaStream_t st) {
+  ChunkArgs C{};
+  C.E = solver_extract_args(s);
+  C.hist = s->hist;
+  C.snap = s->snap;
+  C.count = s->snap_count;
+  C.steps = 0;
+  C.max_steps = kSequence;
+  return launch_chunk_extract(C, st);
+}
+
+// A sequence of steps (sequence_length at most), whose sources are there.
+// Beside its stages, on the side stream, the sequence before is extracted and
+// as many sources are built, nbuf / 2 steps ahead.  The stages follow one
+// another directly, each overlapping the tail of the one before; with the
+// fork and join inside every step (and a clock launch and an extraction per
+// step) a step took 2-4 us more: 8192 x 128 62.3 -> 59.5, 4096 x 128 35.3 -> 33.5.
+// A single step extracts itself and then builds its one source.
+static int launch_sequence(bhr_solver *s, int count) {
+  SourceArgs S = solver_source_args(s);
+  if (count == 1) {
+    if (int st = launch_stages(s, 0, false, false)) return st;
+    BHR_CUDA_TRY(launch_extract(solver_extract_args(s), s->stream));
+    S.lookahead = s->nbuf / 2 - 1;  // the clock has been advanced
+    if (s->has_source) BHR_CUDA_TRY(launch_source(S, 1, s->stream));
+    return BHR_OK;
+  }
+  BHR_CUDA_TRY(cudaEventRecord(s->fork, s->stream));
+  BHR_CUDA_TRY(cudaStreamWaitEvent(s->side, s->fork, 0));
+  BHR_CUDA_TRY(launch_extraction(s, s->side));
+  S.lookahead = s->nbuf / 2;
+  if (s->has_source) BHR_CUDA_TRY(launch_source(S, count, s->side));
+  BHR_CUDA_TRY(cudaEventRecord(s->join, s->side));
+  for (int i = 0; i < count; i++)
+    if (int st = launch_stages(s, i, true, !s->rk4 && (i & 1))) return st;
+  BHR_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->join, 0));
+  BHR_CUDA_TRY(launch_step_clock(s->rs, count, s->stream));
   return BHR_OK;
 }
 
@@ -1162,21 +1205,15 @@ static int check_run_state(bhr_solver *s) {
   return BHR_OK;
 }
 
-// Captures `count` steps of launch_step into an executable graph.  Every
-// launch argument is fixed per solve; what changes from step to step (the
-// step clocks, the timer, the source record) is read on the device from
-// RunState, so one captured graph replays any step.  A graph starts and ends
-// with an extraction pending: it extracts the step before it and leaves its
-// own last step's extraction to what follows.
-static int capture_steps(bhr_solver *s, int count, cudaGraphExec_t *out) {
+// Captures a sequence of steps into an executable graph.  Every launch
+// argument is fixed per solve; what changes from step to step (the step
+// clocks, the timer, the source record) is read on the device from RunState,
+// so one captured graph replays any sequence.
+static int capture_sequence(bhr_solver *s, int count, cudaGraphExec_t *out) {
   cudaGraph_t g = nullptr;
-  const bool pending = s->pending_extract;
-  s->pending_extract = true;
   BHR_CUDA_TRY(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-  int st = BHR_OK;
-  for (int i = 0; i < count && st == BHR_OK; i++) st = launch_step(s, nullptr, !s->rk4 && (i & 1));
+  const int st = launch_sequence(s, count);
   cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-  s->pending_extract = pending;
   if (st != BHR_OK) {
     if (g) cudaGraphDestroy(g);
     return st;
@@ -1199,7 +1236,6 @@ static int capture_steps(bhr_solver *s, int count, cudaGraphExec_t *out) {
 // the device has no room for a cooperative launch: the caller steps by stage).
 static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
   *done = 0;
-  if (int st = flush_extract(s)) return st;
   const StageArgs A = solver_stage_args(s);
   ResidentArgs R{};
   R.u = s->u0;
@@ -1215,10 +1251,7 @@ static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
   R.strips = s->rgeom.strips;
   R.segs = s->rgeom.segs;
   R.rmax = s->rgeom.rmax;
-  // the extraction column, or the two interior columns its closure reads
-  const int a = s->ext_col, N = s->p.N;
-  R.ext[0] = a < 3 ? 3 : a >= N - 3 ? N - 4 : a;
-  R.ext[1] = a < 3 ? 4 : a >= N - 3 ? N - 5 : -1;
+  history_columns(s, R.ext);
   R.dt = A.dt;
   R.cx = A.cx;
   R.cy = A.cy;
@@ -1232,7 +1265,7 @@ static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
   C.snap = s->snap;
   C.count = s->snap_count;
   while (*done < nsteps) {
-    R.steps = C.steps = std::min(kResidentChunk, nsteps - *done);
+    R.steps = C.steps = C.max_steps = std::min(kResidentChunk, nsteps - *done);
     R.seq = s->rseq;
     const cudaError_t e = launch_resident(R, s->stream);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
@@ -1249,6 +1282,18 @@ static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
   return BHR_OK;
 }
 
+// The graphs a call of nsteps by stage will use: of one step for calls of one
+// step, of a full sequence for long runs.
+static int prepare_graphs(bhr_solver *s, int nsteps) {
+  if (s->resident && !s->has_source) return BHR_OK;
+  if (nsteps == 1 && !s->g1) return capture_sequence(s, 1, &s->g1);
+  const int length = sequence_length(s);
+  const bool graph = s->nt - s->steps_done >= kGraphSteps || static_cast<size_t>(s->p.N) * s->p.M < kDirectPoints;
+  if (length > 1 && nsteps >= length && graph && !s->gb)
+    return capture_sequence(s, length, &s->gb);
+  return BHR_OK;
+}
+
 static int enqueue_steps(bhr_solver *s, int nsteps) {
   if (nsteps <= 0) return BHR_OK;
   if (s->resident && !s->has_source) {
@@ -1257,20 +1302,26 @@ static int enqueue_steps(bhr_solver *s, int nsteps) {
     nsteps -= done;
     if (nsteps <= 0) return BHR_OK;
   }
-  if (!s->g1)
-    if (int st = capture_steps(s, 1, &s->g1)) return st;
-  if (nsteps >= kGraphBatch && !s->gb)
-    if (int st = capture_steps(s, kGraphBatch, &s->gb)) return st;
-  int left = nsteps;
-  if (!s->pending_extract) {  // the graphs start with an extraction pending
-    if (int st = launch_step(s)) return st;
-    left--;
+  if (int st = prepare_graphs(s, nsteps)) return st;
+  const int length = sequence_length(s);
+  bool pending = false;  // a sequence has run and is not extracted
+  for (int left = nsteps; left > 0;) {
+    const int n = std::min(left, length);
+    if (n == 1 && pending) {
+      BHR_CUDA_TRY(launch_extraction(s, s->stream));
+      pending = false;
+    }
+    if (n > 1) pending = true;
+    if (n == 1 && s->g1) {
+      BHR_CUDA_TRY(cudaGraphLaunch(s->g1, s->stream));
+    } else if (n == length && s->gb) {
+      BHR_CUDA_TRY(cudaGraphLaunch(s->gb, s->stream));
+    } else if (int st = launch_sequence(s, n)) {
+      return st;
+    }
+    left -= n;
   }
-  while (left >= kGraphBatch) {
-    BHR_CUDA_TRY(cudaGraphLaunch(s->gb, s->stream));
-    left -= kGraphBatch;
-  }
-  while (left-- > 0) BHR_CUDA_TRY(cudaGraphLaunch(s->g1, s->stream));
+  if (pending) BHR_CUDA_TRY(launch_extraction(s, s->stream));
   s->steps_done += nsteps;
   return BHR_OK;
 }
@@ -1285,7 +1336,7 @@ int bhr_solver_step(bhr_solver *s, int nsteps) {
     set_error("stepping past the end of the trajectory records");
     return BHR_INVALID_ARG;
   }
-  if (int st = solver_wait_records(s, s->steps_done + nsteps + 1)) return st;
+  if (int st = solver_wait_records(s, s->steps_done + nsteps + 1, s->nbuf / 2)) return st;
   if (int st = enqueue_steps(s, nsteps)) return st;
   return check_run_state(s);
 }
@@ -1298,12 +1349,8 @@ int bhr_solver_time_steps(bhr_solver *s, int nsteps, double *ms) {
     set_error("stepping past the end of the trajectory records");
     return BHR_INVALID_ARG;
   }
-  if (int st = solver_wait_records(s, s->steps_done + nsteps + 1)) return st;
-  const bool graphs = !s->resident || s->has_source;
-  if (graphs && !s->g1)
-    if (int st = capture_steps(s, 1, &s->g1)) return st;
-  if (graphs && nsteps >= kGraphBatch && !s->gb)
-    if (int st = capture_steps(s, kGraphBatch, &s->gb)) return st;
+  if (int st = solver_wait_records(s, s->steps_done + nsteps + 1, s->nbuf / 2)) return st;
+  if (int st = prepare_graphs(s, nsteps)) return st;
   cudaEvent_t e0, e1;
   BHR_CUDA_TRY(cudaEventCreate(&e0));
   BHR_CUDA_TRY(cudaEventCreate(&e1));
@@ -1323,7 +1370,6 @@ int bhr_solver_time_steps(bhr_solver *s, int nsteps, double *ms) {
 int bhr_solver_waveform(bhr_solver *s, double *t, double *h, double *dedt, int max_rows, int *nrows) {
   if (!s) return BHR_INVALID_ARG;
   BHR_CUDA_TRY(cudaSetDevice(s->p.device));
-  if (int st = flush_extract(s)) return st;
   RunState rs{};
   BHR_CUDA_TRY(cudaMemcpyAsync(&rs, s->rs, sizeof(rs), cudaMemcpyDeviceToHost, s->stream));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -1351,7 +1397,6 @@ int bhr_solver_run(bhr_solver *s, const char *out_dir, const char *name) {
   for (int done = 0; done < remaining; done += chunk) {
     if (int st = bhr_solver_step(s, std::min(chunk, remaining - done))) return st;
   }
-  if (int st = flush_extract(s)) return st;
   if (int st = check_run_state(s)) return st;
   if (!out_dir || !name) return BHR_OK;
   RunState rs{};
@@ -1401,7 +1446,6 @@ int bhr_write_waveform(const char *out_dir, const char *name, double m, const do
 int bhr_solver_get_state(bhr_solver *s, double *qre, double *qim, double *pre, double *pim) {
   if (!s) return BHR_INVALID_ARG;
   BHR_CUDA_TRY(cudaSetDevice(s->p.device));
-  if (int st = flush_extract(s)) return st;
   const size_t NM = static_cast<size_t>(s->p.N) * s->p.M;
   BHR_CUDA_TRY(launch_closure(s->u0, s->p.N, s->p.M, s->even_m ? 1 : 0, s->stream));
   double *outs[4] = {qre, qim, pre, pim};
@@ -1414,7 +1458,6 @@ int bhr_solver_get_state(bhr_solver *s, double *qre, double *qim, double *pre, d
 int bhr_solver_set_state(bhr_solver *s, const double *qre, const double *qim, const double *pre, const double *pim) {
   if (!s) return BHR_INVALID_ARG;
   BHR_CUDA_TRY(cudaSetDevice(s->p.device));
-  if (int st = flush_extract(s)) return st;
   const size_t NM = static_cast<size_t>(s->p.N) * s->p.M;
   const double *ins[4] = {qre, qim, pre, pim};
   for (int f = 0; f < 4; f++) {
@@ -1429,7 +1472,6 @@ int bhr_solver_get_extraction(bhr_solver *s, double *psi_re, double *psi_im, dou
                               double *dint_re, double *dint_im) {
   if (!s) return BHR_INVALID_ARG;
   BHR_CUDA_TRY(cudaSetDevice(s->p.device));
-  if (int st = flush_extract(s)) return st;
   const int M = s->p.M;
   std::vector<double> e(2 * M), in(4 * M);
   BHR_CUDA_TRY(cudaMemcpyAsync(e.data(), s->ext, e.size() * 8, cudaMemcpyDeviceToHost, s->stream));
@@ -1468,7 +1510,6 @@ extern "C" {
 int bhr_solver_psi_samples(bhr_solver *s, double *psi_re, double *psi_im, int max_rows, int *nrows) {
   if (!s) return BHR_INVALID_ARG;
   BHR_CUDA_TRY(cudaSetDevice(s->p.device));
-  if (int st = flush_extract(s)) return st;
   RunState rs{};
   BHR_CUDA_TRY(cudaMemcpyAsync(&rs, s->rs, sizeof(rs), cudaMemcpyDeviceToHost, s->stream));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
@@ -1490,7 +1531,6 @@ int bhr_solver_psi_samples(bhr_solver *s, double *psi_re, double *psi_im, int ma
 size_t bhr_solver_checkpoint_size(bhr_solver *s) {
   if (!s) return 0;
   cudaSetDevice(s->p.device);
-  if (flush_extract(s)) return 0;
   RunState rs{};
   if (cudaMemcpyAsync(&rs, s->rs, sizeof(rs), cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||
       cudaStreamSynchronize(s->stream) != cudaSuccess)
@@ -1502,7 +1542,6 @@ int bhr_solver_checkpoint(bhr_solver *s, void *buf, size_t size) {
   NvtxRange range("bhr_solver_checkpoint");
   if (!s || !buf) return BHR_INVALID_ARG;
   BHR_CUDA_TRY(cudaSetDevice(s->p.device));
-  if (int st = flush_extract(s)) return st;
   CheckpointHeader h{};
   std::memcpy(h.magic, kCkptMagic, sizeof(h.magic));
   BHR_CUDA_TRY(cudaMemcpyAsync(&h.rs, s->rs, sizeof(RunState), cudaMemcpyDeviceToHost, s->stream));
@@ -1550,9 +1589,8 @@ int bhr_solver_restore(bhr_solver *s, const void *buf, size_t size) {
     set_error("checkpoint does not match this solve (grid, spin, m, dt, length or trajectory)");
     return BHR_INVALID_ARG;
   }
-  if (int st = flush_extract(s)) return st;
   if (s->has_source)
-    if (int st = solver_wait_records(s, h.rs.ks + 1)) return st;
+    if (int st = solver_wait_records(s, h.rs.ks + 1, s->nbuf / 2)) return st;
   const size_t NM = static_cast<size_t>(s->p.N) * s->p.M, M = s->p.M;
   const double *d = reinterpret_cast<const double *>(static_cast<const char *>(buf) + sizeof(h));
   BHR_CUDA_TRY(cudaMemcpyAsync(s->u0, d, 4 * NM * 8, cudaMemcpyHostToDevice, s->stream));
@@ -1565,8 +1603,8 @@ int bhr_solver_restore(bhr_solver *s, const void *buf, size_t size) {
                                  2 * M * static_cast<size_t>(h.rs.nrow) * 8, cudaMemcpyHostToDevice, s->stream));
   }
   BHR_CUDA_TRY(cudaMemcpyAsync(s->rs, &h.rs, sizeof(RunState), cudaMemcpyHostToDevice, s->stream));
-  // The patch of the step the solve resumes at (later ones are built ahead).
-  if (s->has_source) BHR_CUDA_TRY(launch_source(solver_source_args(s), s->stream));
+  // The patches of the sequence the solve resumes with.
+  if (s->has_source) BHR_CUDA_TRY(launch_first_sources(s));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
   s->steps_done = h.steps_done;
   return BHR_OK;
@@ -1587,7 +1625,7 @@ int bhr_solver_get_source(bhr_solver *s, double *tre, double *tim) {
   StepRec rec{};
   std::vector<double> patch(2 * static_cast<size_t>(p.PTSX) * p.PTSY);
   BHR_CUDA_TRY(cudaMemcpyAsync(&rec, s->recs + (rs.ks - 1), sizeof(rec), cudaMemcpyDeviceToHost, s->stream));
-  BHR_CUDA_TRY(cudaMemcpyAsync(patch.data(), s->src + ((rs.ks - 1) & 1) * patch.size(), patch.size() * 8,
+  BHR_CUDA_TRY(cudaMemcpyAsync(patch.data(), s->src + ((rs.ks - 1) % s->nbuf) * patch.size(), patch.size() * 8,
                                cudaMemcpyDeviceToHost, s->stream));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
   for (int j = 0; j < p.PTSY; j++) {
@@ -1613,52 +1651,40 @@ int bhr_solver_profile(bhr_solver *s, int nsteps, double *avg_ms5, double *total
     set_error("profiling past the end of the trajectory records");
     return BHR_INVALID_ARG;
   }
-  if (int st = solver_wait_records(s, s->steps_done + nsteps + 1)) return st;
-  // Events bracket each launch of launch_step; the extraction and the
-  // source run on the side stream beside the stages.
-  std::vector<cudaEvent_t> ev(10 * static_cast<size_t>(nsteps));
+  if (int st = solver_wait_records(s, s->steps_done + nsteps + 1, s->nbuf / 2)) return st;
+  // Events around each kernel of single steps, in the order they run.
+  std::vector<cudaEvent_t> ev(6 * static_cast<size_t>(nsteps));
   for (auto &e : ev) BHR_CUDA_TRY(cudaEventCreate(&e));
-  std::vector<char> had_extract(nsteps);
   double sums[5] = {0, 0, 0, 0, 0};
-  int nextract = 0;
   cudaEvent_t t0, t1;
   BHR_CUDA_TRY(cudaEventCreate(&t0));
   BHR_CUDA_TRY(cudaEventCreate(&t1));
   BHR_CUDA_TRY(cudaEventRecord(t0, s->stream));
   for (int i = 0; i < nsteps; i++) {
-    had_extract[i] = s->pending_extract;
-    if (int st = launch_step(s, &ev[10 * static_cast<size_t>(i)])) return st;
+    cudaEvent_t *e = &ev[6 * static_cast<size_t>(i)];
+    BHR_CUDA_TRY(cudaEventRecord(e[0], s->stream));
+    SourceArgs S = solver_source_args(s);
+    S.lookahead = s->nbuf / 2;
+    if (s->has_source) BHR_CUDA_TRY(launch_source(S, 1, s->stream));
+    if (int st = launch_stages(s, 0, false, false, e + 1)) return st;
+    BHR_CUDA_TRY(launch_extract(solver_extract_args(s), s->stream));
+    BHR_CUDA_TRY(cudaEventRecord(e[5], s->stream));
     s->steps_done++;
   }
   BHR_CUDA_TRY(cudaEventRecord(t1, s->stream));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
-  BHR_CUDA_TRY(cudaStreamSynchronize(s->side));
-  for (int i = 0; i < nsteps; i++) {
-    cudaEvent_t *e = &ev[10 * static_cast<size_t>(i)];
-    float ms = 0.f;
-    if (s->has_source) {
-      BHR_CUDA_TRY(cudaEventElapsedTime(&ms, e[8], e[9]));
-      sums[0] += ms;
-    }
-    for (int j = 1; j < 4; j++) {
-      BHR_CUDA_TRY(cudaEventElapsedTime(&ms, e[j], e[j + 1]));
+  for (int i = 0; i < nsteps; i++)
+    for (int j = s->has_source ? 0 : 1; j < 5; j++) {
+      float ms = 0.f;
+      BHR_CUDA_TRY(cudaEventElapsedTime(&ms, ev[6 * static_cast<size_t>(i) + j], ev[6 * static_cast<size_t>(i) + j + 1]));
       sums[j] += ms;
     }
-    if (had_extract[i]) {
-      BHR_CUDA_TRY(cudaEventElapsedTime(&ms, e[6], e[7]));
-      sums[4] += ms;
-      nextract++;
-    }
-  }
   float tot = 0.f;
   BHR_CUDA_TRY(cudaEventElapsedTime(&tot, t0, t1));
   for (auto &e : ev) cudaEventDestroy(e);
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
-  if (avg_ms5) {
-    for (int j = 0; j < 4; j++) avg_ms5[j] = sums[j] / nsteps;
-    avg_ms5[4] = nextract ? sums[4] / nextract : 0.0;
-  }
+  for (int j = 0; avg_ms5 && j < 5; j++) avg_ms5[j] = sums[j] / nsteps;
   if (total_ms) *total_ms = tot;
   return check_run_state(s);
 }

@@ -18,10 +18,11 @@ struct bhr_solver {
   bool even_m = true;
   bool has_source = false;
   cudaStream_t stream = nullptr;
-  // The particle source of step k+1 is built on `side` while step k's
-  // stages run: forked after step k-1's extraction, joined into step k's.
+  // Beside the stages of a sequence of steps, the sources of the next one are
+  // built and the one before is extracted on `side`, forked at the sequence's
+  // start and joined at its end.
   cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr, fork2 = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   // device memory
   double *u0 = nullptr, *u1 = nullptr, *u2 = nullptr;
   // classical RK4 (BHR_RK4): u1 holds y1 then y3, u2 y2, u3 z = (y1 + 2 y2 - u^n)/3
@@ -29,6 +30,9 @@ struct bhr_solver {
   double *u3 = nullptr;
   double *coltab = nullptr, *rowtab = nullptr, *ctab = nullptr, *rc = nullptr, *th = nullptr;
   double *src = nullptr, *ext = nullptr, *integ = nullptr, *wproj = nullptr, *wdedt = nullptr, *rows = nullptr;
+  // a sequence's extraction columns and output snapshots
+  double *hist = nullptr, *snap = nullptr;
+  int *snap_count = nullptr;
   double *psirows = nullptr;  // psi(theta) at the extraction column per waveform row
   // mixed precision (BHR_MIXED): FP32 delta1 and eps2 planes, FP32 tables
   bool mixed = false;
@@ -53,14 +57,10 @@ struct bhr_solver {
   bool resident = false;
   bhr::ResidentGeom rgeom{};
   ulonglong2 *inbox = nullptr;   // edge words of the blocks
-  double *hist = nullptr, *snap = nullptr;  // a launch's extraction columns and output snapshots
-  int *snap_count = nullptr;
   unsigned long long rseq = 1;   // number of the next launch's first edge words
   int steps_done = 0;
-  // The extraction of the last step launched has not been launched yet: it
-  // runs beside the next step's first stages, or before a host read.
-  bool pending_extract = false;
-  // Captured step graphs: one step, and kGraphBatch steps in one launch.
+  int nbuf = 2;        // source patch buffers
+  // Captured graphs: one step, and a full sequence of steps.
   cudaGraphExec_t g1 = nullptr, gb = nullptr;
   // Per-step source records past the first chunk are built and uploaded by
   // a host thread after set_trajectory returns; stepping waits for the
@@ -88,6 +88,8 @@ SourceArgs solver_source_args(bhr_solver *s);
 ExtractArgs solver_extract_args(bhr_solver *s);
 MixedArgs solver_mixed_args(bhr_solver *s);
 // Waits until the source records of steps [0, upto) are on the device
-// (returns the status of a record that failed before upto).
-int solver_wait_records(bhr_solver *s, int upto);
+// (returns the status of a record that failed before upto), then for `ahead`
+// more unless they fail or end (patches are built that far ahead; those of
+// steps that cannot run are not read).
+int solver_wait_records(bhr_solver *s, int upto, int ahead = 0);
 }  // namespace bhr
