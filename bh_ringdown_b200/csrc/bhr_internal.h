@@ -178,24 +178,30 @@ cudaError_t launch_stage12_strip(const StripMaps &maps, const StageArgs &a, cuda
 // one 64-column tile of up to kResidentMaxRows rows per block, strips x segs
 // blocks.  ok is false for grids that do not fit (more strips than SMs, or
 // taller tiles).
-constexpr int kResidentMaxRows = 32;
+constexpr int kResidentMaxRows = 32;     // FP64 SSP-RK3 without a source
+constexpr int kResidentSourceRows = 16;  // with one
+constexpr int kResidentRk4Rows = 16;     // RK4: z's planes take the room of the taller tile
 constexpr int kResidentChunk = 64;  // steps per launch
 struct ResidentGeom {
   int strips, segs, rmax;
   bool ok;
 };
-ResidentGeom resident_geometry(int N, int M);
+ResidentGeom resident_geometry(int N, int M, bool rk4 = false);
 size_t resident_inbox_bytes(const ResidentGeom &g);
 struct ResidentArgs {
   double *u;             // state planes, advanced in place
   const double *coltab, *rowtab, *bb;
-  ulonglong2 *inbox;     // resident_inbox_bytes, no word numbered seq .. seq + 3 steps - 1 yet
+  ulonglong2 *inbox;     // resident_inbox_bytes, no word numbered seq or above yet
   int *err;
   double *hist;          // [steps][2][2][M]: psi_re, psi_im at columns ext[0], ext[1], or nullptr
   unsigned long long seq;  // number of the first stage's edge words
   int N, M, even_m, strips, segs, rmax, steps;
   int ext[2];            // columns recorded (-1: none)
   int close;             // 1: also write the closure of the boundary rows and columns
+  int rk4;               // 1: classical RK4 (four stages a step)
+  const double *src;     // source patches [nbuf][2][PTSY][PTSX] (step k: k % nbuf), or nullptr
+  const StepRec *recs;
+  int ks, nbuf, PTSX, PTSY;  // ks: the first step's number
   double dt, cx, cy, cyy, cko, a2, m4a;
 };
 // Extraction of a sequence of steps: snapshots of the time integrals on

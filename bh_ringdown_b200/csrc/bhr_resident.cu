@@ -1,4 +1,4 @@
-// bhr_resident.cu -- whole SSP-RK3 steps of a small grid in one launch.
+// bhr_resident.cu -- whole SSP-RK3 or RK4 steps of a small grid in one launch.
 //
 // Grids up to ~300 000 points fit in the SMs' shared memory.  Advanced with
 // three launches a step they are bound by launch latency and by refetching
@@ -18,6 +18,12 @@
 // Measured on 148 SMs, us per step (three stages), stage launches -> here:
 // 256 x 32 10.4 -> 5.2, 1024 x 64 12.7 -> 6.2, 2048 x 64 14.8 -> 10.0,
 // 2048 x 96 21.0 -> 19.1, 2048 x 128 23.2 -> 21.6, 4096 x 64 22.7 -> 20.8.
+// With a source (the patches of a launch's steps are built before it: 0.5 us a
+// step) 512 x 32 13.1 -> 5.8, 1024 x 64 11.7 -> 6.8, 2048 x 64 15.2 -> 10.7;
+// RK4 512 x 32 14.0 -> 6.7, 1024 x 64 15.1 -> 7.9, 1536 x 64 20.1 -> 11.0.
+// Taller tiles with a source lose to the stage launches, which build sources
+// beside the stages (2048 x 128 22.5 there, 23.7 here; 1152 x 256 23.2, 24.1),
+// and RK4's z takes their shared memory: both stop at 16 rows.
 // At 1024 x 64 (7-row tiles) 4.5 us of the 6.2 are a lone row's instruction
 // stream (latency of FP64 and shared-memory chains with 3-4 warps a
 // scheduler), 1.4 us waiting for edges; from 9 rows on the FP64 issue rate
@@ -67,12 +73,13 @@ __device__ __forceinline__ ulonglong2 edge_load(const ulonglong2 *slot) {
 __host__ __device__ constexpr int res_rows(int cols, int rpw) { return kResWarps * rpw * cols / 2; }
 // Shared memory (doubles), laid out for a shape's tallest tile R so that every
 // stride is a constant: q [2 buffers][2][R + 6][WC], p [1 or 2 buffers][2][R]
-// [WC] (a row of one warp is updated in place), u^n [4][R][TC] and, where a
-// warp has several rows, bb [R][WC], row factors [R][RF_COUNT] and column
-// factors [CF_TILE][TC].
-__host__ __device__ constexpr int res_smem_doubles(int cols, int rpw) {
+// [WC] (a row of one warp is updated in place), u^n [4][R][TC], RK4's z
+// [4][R][TC] and, where a warp has several rows, bb [R][WC], row factors [R]
+// [RF_COUNT] and column factors [CF_TILE][TC].
+__host__ __device__ constexpr int res_smem_doubles(int cols, int rpw, bool rk4) {
   const int R = res_rows(cols, rpw);
-  return 4 * (R + 6) * WC + (cols == 1 ? 4 : 2) * R * WC + 4 * R * TC + (rpw == 1 ? 0 : R * WC + R * RF_COUNT + CF_TILE * TC);
+  return 4 * (R + 6) * WC + (cols == 1 ? 4 : 2) * R * WC + (rk4 ? 8 : 4) * R * TC +
+         (rpw == 1 ? 0 : R * WC + R * RF_COUNT + CF_TILE * TC);
 }
 // A block's inbox, 16-byte words: q rows from above and below [2 planes][3]
 // [TC] each, q columns from the left and the right [2 planes][rmax][4] each,
@@ -152,12 +159,16 @@ __device__ __forceinline__ void pole(double (&g)[COLS], const double (&g1)[COLS]
 }
 
 // With one row per warp a thread keeps its points' coefficients in registers
-// for the whole launch; with two they are formed again each stage.
-template <int COLS, int RPW>
+// for the whole launch; with two they are formed again each stage.  SRC: the
+// solve has a particle source (each step's patch read from memory).  RK4:
+// classical RK4 instead of SSP-RK3, its stages combined as the stage kernels
+// combine them (one row per warp only: z takes the shared memory).
+template <int COLS, int RPW, bool SRC, bool RK4>
 __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_constant__ ResidentArgs A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int abort_flag;
   constexpr bool KEEP = RPW == 1;
+  constexpr int STAGES = RK4 ? 4 : 3;
   constexpr int PBUFS = COLS == 1 ? 2 : 1;
   // q edge words a thread receives: (768 + 16 rows) / 512
   constexpr int kSlots = (12 * TC + 16 * res_rows(COLS, RPW) + kResThreads - 1) / kResThreads;
@@ -169,7 +180,8 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
   const bool has_l = strip > 0, has_r = strip + 1 < A.strips, has_t = seg > 0, has_b = seg + 1 < A.segs;
   constexpr int RS = res_rows(COLS, RPW), qpl = (RS + 6) * WC, ppl = RS * WC;  // rows laid out, plane strides
   double *const q0 = reinterpret_cast<double *>(smem_raw), *const p0 = q0 + 4 * qpl, *const un = p0 + 2 * PBUFS * ppl,
-                *const bbs = un + 4 * RS * TC, *const rowf = bbs + RS * WC, *const colf = rowf + RS * RF_COUNT;
+                *const zn = un + 4 * RS * TC, *const bbs = RK4 ? zn + 4 * RS * TC : zn,
+                *const rowf = bbs + RS * WC, *const colf = rowf + RS * RF_COUNT;
   const int row0 = COLS == 2 ? warp : warp >> 1;                        // this warp's first row
   const int col = COLS == 2 ? 2 * lane : 32 * (warp & 1) + lane;        // this thread's first column in the tile
   const int a0 = c0 + col, w0 = col + 4;
@@ -312,24 +324,41 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
   const double d1a = 45.0 * A.cx, d1b = -9.0 * A.cx, d1c_ = A.cx;
   const double y2a = -490.0 * A.cyy, y2b = 270.0 * A.cyy, y2c = -27.0 * A.cyy, y2d = 2.0 * A.cyy;
   const double pole_w = A.even_m ? kThird : 0.0;
+  // cq f + cu u, with the terms the weights (constants once unrolled) take out left out.
+  auto combine = [](const double cq, const double f, const double cu, const double u) {
+    return cu == 0.0 ? f : cq == 0.0 ? u : cu == 1.0 ? fma(cq, f, u) : fma(cq, f, cu * u);
+  };
   unsigned long long seq = A.seq;
   bool aborted = false, first = true;
   int cur = 0;  // buffer of the stage input
 
 #pragma unroll 1
   for (int step = 0; step < A.steps; step++) {
+    // The step's source patch: this thread's first column and the tile's
+    // first row in it.
+    int src_c = 0, src_r = 0;
+    const double *patch = nullptr;
+    if (SRC) {
+      const int k = A.ks + step;
+      src_c = a0 - __ldg(&A.recs[k].col0);
+      src_r = b0 - __ldg(&A.recs[k].row0);
+      patch = A.src + static_cast<size_t>(k % A.nbuf) * 2 * A.PTSX * A.PTSY;
+    }
 #pragma unroll
-    for (int stage = 1; stage <= 3; stage++, seq++) {
-      const bool last = stage == 3 && step + 1 == A.steps;
+    for (int stage = 1; stage <= STAGES; stage++, seq++) {
+      const bool last = stage == STAGES && step + 1 == A.steps;
       const int par = static_cast<int>(seq & 1) * words, par0 = words - par;  // this stage's words, the input's
       const double *q = q0 + cur * 2 * qpl;
       double *qn = q0 + (cur ^ 1) * 2 * qpl;
       double *p = p0 + (PBUFS == 2 ? cur * 2 * ppl : 0), *pn = p0 + (PBUFS == 2 ? (cur ^ 1) * 2 * ppl : 0);
-      // The stage combination cu u^n + cf f + cr L (HighOrder/kern.cu:
-      // 301-318, 582-620; the weights as the reference rounds them).
-      const double cu = stage == 1 ? 0.0 : stage == 2 ? 0.75 : kThird;
-      const double cq = stage == 1 ? 1.0 : stage == 2 ? 0.25 : 2.0 * kThird;
-      const double cr = cq * A.dt;
+      // The stage combination cu u^n + cq f + cr L (HighOrder/kern.cu:
+      // 301-318, 582-620; the weights as the reference rounds them).  RK4:
+      // u + dt/2 L, u + dt/2 L, u + dt L, z + y3/3 + dt/6 L.
+      const double cu = RK4 ? (stage == 1 ? 0.0 : 1.0) : stage == 1 ? 0.0 : stage == 2 ? 0.75 : kThird;
+      const double cq = RK4 ? (stage == 1 ? 1.0 : stage == 4 ? kThird : 0.0)
+                            : stage == 1 ? 1.0 : stage == 2 ? 0.25 : 2.0 * kThird;
+      const double cr = RK4 ? (stage < 3 ? 0.5 * A.dt : stage == 3 ? A.dt : A.dt / 6.0) : cq * A.dt;
+      const double *us = RK4 && stage == 4 ? zn : un;
 #pragma unroll 1
       for (int i = 0; i < RPW; i++) {
         const int r = row0 + i * kResWarps, b = b0 + r;
@@ -339,6 +368,19 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
         const ulonglong2 *p_in = A.inbox + T.p_word + par0;
         ulonglong2 pw = make_ulonglong2(0, 0);
         if (T.p_word >= 0) pw = edge_load(p_in);
+        // The source at its points, likewise.
+        double sv[2][COLS];
+        if (SRC) {
+          const int sr = src_r + r;
+          const bool on = sr >= 0 && sr < A.PTSY;
+#pragma unroll
+          for (int c = 0; c < COLS; c++) {
+            const bool in = on && src_c + c >= 0 && src_c + c < A.PTSX;
+            const double *x = patch + static_cast<size_t>(sr) * A.PTSX + src_c + c;
+            sv[0][c] = in ? __ldg(x) : 0.0;
+            sv[1][c] = in ? __ldg(x + static_cast<size_t>(A.PTSY) * A.PTSX) : 0.0;
+          }
+        }
         if (!KEEP) {
           double w[6 + COLS], cf[CF_TILE][COLS];
 #pragma unroll
@@ -370,7 +412,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
             pole<COLS>(g[6], g[5], g[4], pole_w);
           }
           double u[COLS];
-          get<COLS>(u, un + (pl * RS + r) * TC + col);
+          get<COLS>(u, us + (pl * RS + r) * TC + col);
 #pragma unroll
           for (int c = 0; c < COLS; c++) {
             // Theta derivatives (HighOrder/kern.cu:206-226).
@@ -382,7 +424,8 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
             const double fx = fma(d1a, v[5 + c] - v[3 + c], fma(d1b, v[6 + c] - v[2 + c], d1c_ * (v[7 + c] - v[1 + c])));
             const double kd = fma(-8.0, v[7 + c] + v[1 + c], v[8 + c] + v[c]) +
                               fma(28.0, v[6 + c] + v[2 + c], fma(-56.0, v[5 + c] + v[3 + c], 70.0 * f));
-            o[pl][c] = fma(cr, fma(kon[c], kd, fma(-C.bb[c], fx, pc[pl][c])), fma(cq, f, cu * u[c]));
+            o[pl][c] = fma(cr, fma(kon[c], kd, fma(-C.bb[c], fx, pc[pl][c])), combine(cq, f, cu, u[c]));
+            if (RK4 && stage == 2) zn[(pl * RS + r) * TC + col + c] = (f + 2.0 * o[pl][c] - u[c]) * kThird;
             // the p equation's q terms (HighOrder/kern.cu:281-296)
             if (pl == 0) {
               res[0][c] = fma(C.cc[c], ll, fma(C.dre[c], fx, C.vre[c] * f));
@@ -412,7 +455,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
             for (int e = 0; e < 2 * COLS; e++) edge_send(s + (e / COLS) * 4 * A.rmax + e % COLS, o[e / COLS][e % COLS], seq);
           }
         }
-        if (stage == 3) {
+        if (stage == STAGES) {
 #pragma unroll
           for (int pl = 0; pl < 2; pl++) {
             put<COLS>(un + (pl * RS + r) * TC + col, o[pl]);
@@ -457,7 +500,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
         for (int pl = 0; pl < 2; pl++) {
           double v[8 + COLS], u[COLS];
           window<COLS>(v, p + pl * ppl + r * WC + w0, pc[pl]);
-          get<COLS>(u, un + ((2 + pl) * RS + r) * TC + col);
+          get<COLS>(u, us + ((2 + pl) * RS + r) * TC + col);
 #pragma unroll
           for (int c = 0; c < COLS; c++) {
             const double fx = fma(d1a, v[5 + c] - v[3 + c], fma(d1b, v[6 + c] - v[2 + c], d1c_ * (v[7 + c] - v[1 + c])));
@@ -465,7 +508,9 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
                               fma(28.0, v[6 + c] + v[2 + c], fma(-56.0, v[5 + c] + v[3 + c], 70.0 * v[4 + c]));
             const double t = pl == 0 ? fma(C.are[c], pc[0][c], fma(-C.aim[c], pc[1][c], res[0][c]))
                                      : fma(C.are[c], pc[1][c], fma(C.aim[c], pc[0][c], res[1][c]));
-            o[pl][c] = fma(cr, fma(C.ee[c], fx, fma(kon[c], kd, t)), fma(cq, v[4 + c], cu * u[c]));
+            const double x = SRC ? t + sv[pl][c] : t;
+            o[pl][c] = fma(cr, fma(C.ee[c], fx, fma(kon[c], kd, x)), combine(cq, v[4 + c], cu, u[c]));
+            if (RK4 && stage == 2) zn[((2 + pl) * RS + r) * TC + col + c] = (v[4 + c] + 2.0 * o[pl][c] - u[c]) * kThird;
           }
         }
         if (PBUFS == 1) __syncwarp();  // the row has been read
@@ -476,7 +521,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
 #pragma unroll
           for (int e = 0; e < 2 * COLS; e++) edge_send(s + (e / COLS) * 4 + e % COLS, o[e / COLS][e % COLS], seq);
         }
-        if (stage == 3) {
+        if (stage == STAGES) {
 #pragma unroll
           for (int pl = 0; pl < 2; pl++) {
             put<COLS>(un + ((2 + pl) * RS + r) * TC + col, o[pl]);
@@ -685,14 +730,14 @@ __global__ void __launch_bounds__(kChunkThreads) chunk_project_kernel(const __gr
 
 }  // namespace
 
-ResidentGeom resident_geometry(int N, int M) {
+ResidentGeom resident_geometry(int N, int M, bool rk4) {
   ResidentGeom g{};
   const int sms = device_sm_count(), rows = M - 6;
   g.strips = N / TC;
   if (g.strips > sms) return g;
   g.segs = std::max(1, std::min(sms / g.strips, rows / 3));  // a neighbour's halo comes from one tile: 3 rows at least
   g.rmax = (rows + g.segs - 1) / g.segs;
-  g.ok = rows / g.segs >= 3 && g.rmax <= kResidentMaxRows;
+  g.ok = rows / g.segs >= 3 && g.rmax <= (rk4 ? kResidentRk4Rows : kResidentMaxRows);
   return g;
 }
 
@@ -700,14 +745,30 @@ size_t resident_inbox_bytes(const ResidentGeom &g) {
   return static_cast<size_t>(g.strips) * g.segs * 2 * res_inbox_words(g.rmax) * 16;
 }
 
+// f(kernel, shared memory bytes) for the kernel of a shape, source and
+// integrator.
+template <class F>
+static cudaError_t with_resident_kernel(int rmax, bool src, bool rk4, F &&f) {
+  auto bytes = [&](int cols, int rpw) { return static_cast<int>(sizeof(double)) * res_smem_doubles(cols, rpw, rk4); };
+  if (rmax <= res_rows(1, 1)) {
+    if (rk4) return src ? f(resident_kernel<1, 1, true, true>, bytes(1, 1)) : f(resident_kernel<1, 1, false, true>, bytes(1, 1));
+    return src ? f(resident_kernel<1, 1, true, false>, bytes(1, 1)) : f(resident_kernel<1, 1, false, false>, bytes(1, 1));
+  }
+  if (rmax <= res_rows(2, 1)) {
+    if (rk4) return src ? f(resident_kernel<2, 1, true, true>, bytes(2, 1)) : f(resident_kernel<2, 1, false, true>, bytes(2, 1));
+    return src ? f(resident_kernel<2, 1, true, false>, bytes(2, 1)) : f(resident_kernel<2, 1, false, false>, bytes(2, 1));
+  }
+  if (src || rk4 || rmax > kResidentMaxRows) return cudaErrorInvalidValue;
+  return f(resident_kernel<2, 2, false, false>, bytes(2, 2));
+}
+
 cudaError_t prepare_resident_kernels() {
-  constexpr auto kSmem = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t r;
-  auto bytes = [](int cols, int rpw) { return res_smem_doubles(cols, rpw) * 8; };
-  if ((r = cudaFuncSetAttribute(resident_kernel<1, 1>, kSmem, bytes(1, 1))) ||
-      (r = cudaFuncSetAttribute(resident_kernel<2, 1>, kSmem, bytes(2, 1))) ||
-      (r = cudaFuncSetAttribute(resident_kernel<2, 2>, kSmem, bytes(2, 2))))
-    return r;
+  for (int rmax : {res_rows(1, 1), res_rows(2, 1), res_rows(2, 2)})
+    for (int v = 0; v < (rmax <= res_rows(2, 1) ? 4 : 1); v++)
+      if (cudaError_t e = with_resident_kernel(rmax, v & 1, v >> 1, [](auto kernel, int bytes) {
+            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+          }))
+        return e;
   return cudaSuccess;
 }
 
@@ -749,11 +810,8 @@ static cudaError_t launch_cooperative(void (*kernel)(const ResidentArgs), const 
 
 cudaError_t launch_resident(const ResidentArgs &a, cudaStream_t st) {
   if (a.steps <= 0) return cudaSuccess;
-  if (a.rmax > kResidentMaxRows) return cudaErrorInvalidValue;
-  auto bytes = [](int cols, int rpw) { return sizeof(double) * res_smem_doubles(cols, rpw); };
-  if (a.rmax <= res_rows(1, 1)) return launch_cooperative(resident_kernel<1, 1>, a, bytes(1, 1), st);
-  if (a.rmax <= res_rows(2, 1)) return launch_cooperative(resident_kernel<2, 1>, a, bytes(2, 1), st);
-  return launch_cooperative(resident_kernel<2, 2>, a, bytes(2, 2), st);
+  return with_resident_kernel(a.rmax, a.src != nullptr, a.rk4 != 0,
+                              [&](auto kernel, int bytes) { return launch_cooperative(kernel, a, bytes, st); });
 }
 
 cudaError_t launch_chunk_extract(const ChunkArgs &a, cudaStream_t st) {

@@ -160,6 +160,7 @@ double tortoise(double r, double a, double rpl, double rmn) {
 }  // namespace
 
 static int autotune_rows(bhr_solver *s);
+static bool runs_resident(const bhr_solver *s);
 static cudaError_t launch_first_sources(bhr_solver *s);
 
 extern "C" {
@@ -315,7 +316,15 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
   // Patch buffers: this sequence's and the next one's steps, two at least.
   const size_t patch = 2 * static_cast<size_t>(p.PTSX) * p.PTSY;
   const bool engine = tile_rows != 0;  // which steps its solves one by one
-  s->nbuf = engine ? 2 : 2 * static_cast<int>(std::max<size_t>(1, std::min<size_t>(kSequence, kPatchBytes / (16 * patch))));
+  // Not the batch engine's solves, whose tile height the caller fixes, nor
+  // solves whose tiling the environment fixes.
+  const char *fixed = std::getenv("BHR_STAGE_TILING");
+  if (!engine && p.precision == BHR_FP64 && (!fixed || !std::strcmp(fixed, "resident"))) {
+    s->rgeom = resident_geometry(p.N, p.M, p.integrator == BHR_RK4);
+    s->resident = s->rgeom.ok;
+  }
+  const int sequences = s->resident && s->rgeom.rmax <= kResidentSourceRows ? kResidentChunk / 2 : kSequence;
+  s->nbuf = engine ? 2 : 2 * static_cast<int>(std::max<size_t>(1, std::min<size_t>(sequences, kPatchBytes / (16 * patch))));
   // The side stream (sources, extraction: a few blocks beside the stages)
   // gets the device's highest priority, so its blocks take the first SM
   // slots that free up.
@@ -386,26 +395,19 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
       return BHR_CUDA_ERROR;
     }
   }
-  // A small grid's source-free FP64 SSP-RK3 steps run several to a launch
-  // (not the batch engine's solves, whose tile height the caller fixes, nor
-  // solves whose tiling the environment fixes).
-  if (tile_rows == 0 && p.precision == BHR_FP64 && p.integrator == BHR_SSPRK3) {
-    const char *v = std::getenv("BHR_STAGE_TILING");
-    s->rgeom = resident_geometry(p.N, p.M);
-    if (s->rgeom.ok && (!v || !std::strcmp(v, "resident"))) {
-      const size_t words = resident_inbox_bytes(s->rgeom) / sizeof(ulonglong2);
-      if ((st = dalloc(s, &s->inbox, words))) {
-        free_all(s);
-        delete s;
-        return st;
-      }
-      if ((e = cudaMemsetAsync(s->inbox, 0, words * sizeof(ulonglong2), s->stream))) {
-        set_error(std::string("upload: ") + cudaGetErrorString(e));
-        free_all(s);
-        delete s;
-        return BHR_CUDA_ERROR;
-      }
-      s->resident = true;
+  // A small grid's FP64 steps run several to a launch.
+  if (s->resident) {
+    const size_t words = resident_inbox_bytes(s->rgeom) / sizeof(ulonglong2);
+    if ((st = dalloc(s, &s->inbox, words))) {
+      free_all(s);
+      delete s;
+      return st;
+    }
+    if ((e = cudaMemsetAsync(s->inbox, 0, words * sizeof(ulonglong2), s->stream))) {
+      set_error(std::string("upload: ") + cudaGetErrorString(e));
+      free_all(s);
+      delete s;
+      return BHR_CUDA_ERROR;
     }
   }
   if (tile_rows == 0) {
@@ -517,7 +519,7 @@ int bhr_solver_info(const bhr_solver *s, bhr_info *info) {
   info->r_plus = s->g.r_plus;
   info->device_bytes = s->bytes;
   info->tile_rows = s->tile_rows;
-  const bool resident = s->resident && !s->has_source;
+  const bool resident = runs_resident(s);
   info->persistent = s->persist || s->ring || resident;
   info->prefetch_ahead = (s->persist || s->ring || resident) ? 0 : stage_prefetch_ahead(s->ahead);
   info->tiling = resident ? BHR_TILING_RESIDENT
@@ -1142,10 +1144,18 @@ static int launch_stages(bhr_solver *s, int step, bool record, bool flip, cudaEv
   return BHR_OK;
 }
 
-static int sequence_length(const bhr_solver *s) { return s->has_source ? s->nbuf / 2 : kSequence; }
+static int sequence_length(const bhr_solver *s) { return s->has_source ? std::min(kSequence, s->nbuf / 2) : kSequence; }
+
+// A grid that fits runs resident, one with a source where its tiles are of one
+// row a warp (kResidentSourceRows).
+static bool runs_resident(const bhr_solver *s) {
+  return s->resident && (!s->has_source || s->rgeom.rmax <= kResidentSourceRows);
+}
 
 // The patches of a sequence from the current step on, before the first.
+// (A resident solve builds those of a launch ahead of it.)
 static cudaError_t launch_first_sources(bhr_solver *s) {
+  if (runs_resident(s)) return cudaSuccess;
   return launch_source(solver_source_args(s), s->nbuf / 2, s->stream);
 }
 
@@ -1231,9 +1241,11 @@ static int capture_sequence(bhr_solver *s, int count, cudaGraphExec_t *out) {
   return BHR_OK;
 }
 
-// Steps of a resident solve (source-free): up to kResidentChunk a launch,
-// each followed by the extraction of its steps.  *done: steps enqueued (0 when
-// the device has no room for a cooperative launch: the caller steps by stage).
+// Steps of a resident solve: up to kResidentChunk a launch (and no more than
+// there are patch buffers), after their sources and before their extraction --
+// one after another, since the launch holds every SM.  *done: steps enqueued
+// (fewer when the device has no room for a cooperative launch: the caller
+// steps on by stage).
 static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
   *done = 0;
   const StageArgs A = solver_stage_args(s);
@@ -1252,6 +1264,12 @@ static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
   R.segs = s->rgeom.segs;
   R.rmax = s->rgeom.rmax;
   history_columns(s, R.ext);
+  R.rk4 = s->rk4;
+  R.src = A.src;
+  R.recs = A.recs;
+  R.nbuf = A.nbuf;
+  R.PTSX = A.PTSX;
+  R.PTSY = A.PTSY;
   R.dt = A.dt;
   R.cx = A.cx;
   R.cy = A.cy;
@@ -1265,8 +1283,11 @@ static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
   C.snap = s->snap;
   C.count = s->snap_count;
   while (*done < nsteps) {
-    R.steps = C.steps = C.max_steps = std::min(kResidentChunk, nsteps - *done);
+    const int most = s->has_source ? std::min(kResidentChunk, s->nbuf) : kResidentChunk;
+    R.steps = C.steps = C.max_steps = std::min(most, nsteps - *done);
     R.seq = s->rseq;
+    R.ks = s->steps_done;
+    if (s->has_source) BHR_CUDA_TRY(launch_source(solver_source_args(s), R.steps, s->stream));
     const cudaError_t e = launch_resident(R, s->stream);
     if (e == cudaErrorCooperativeLaunchTooLarge) {
       cudaGetLastError();
@@ -1274,7 +1295,7 @@ static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
       return BHR_OK;
     }
     BHR_CUDA_TRY(e);
-    s->rseq += 3 * static_cast<unsigned long long>(R.steps);
+    s->rseq += (s->rk4 ? 4 : 3) * static_cast<unsigned long long>(R.steps);
     BHR_CUDA_TRY(launch_chunk_extract(C, s->stream));
     *done += R.steps;
     s->steps_done += R.steps;
@@ -1285,7 +1306,7 @@ static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
 // The graphs a call of nsteps by stage will use: of one step for calls of one
 // step, of a full sequence for long runs.
 static int prepare_graphs(bhr_solver *s, int nsteps) {
-  if (s->resident && !s->has_source) return BHR_OK;
+  if (runs_resident(s)) return BHR_OK;
   if (nsteps == 1 && !s->g1) return capture_sequence(s, 1, &s->g1);
   const int length = sequence_length(s);
   const bool graph = s->nt - s->steps_done >= kGraphSteps || static_cast<size_t>(s->p.N) * s->p.M < kDirectPoints;
@@ -1296,11 +1317,12 @@ static int prepare_graphs(bhr_solver *s, int nsteps) {
 
 static int enqueue_steps(bhr_solver *s, int nsteps) {
   if (nsteps <= 0) return BHR_OK;
-  if (s->resident && !s->has_source) {
+  if (runs_resident(s)) {
     int done = 0;
     if (int st = enqueue_resident(s, nsteps, &done)) return st;
     nsteps -= done;
     if (nsteps <= 0) return BHR_OK;
+    if (s->has_source) BHR_CUDA_TRY(launch_first_sources(s));
   }
   if (int st = prepare_graphs(s, nsteps)) return st;
   const int length = sequence_length(s);
@@ -1663,15 +1685,14 @@ int bhr_solver_profile(bhr_solver *s, int nsteps, double *avg_ms5, double *total
   for (int i = 0; i < nsteps; i++) {
     cudaEvent_t *e = &ev[6 * static_cast<size_t>(i)];
     BHR_CUDA_TRY(cudaEventRecord(e[0], s->stream));
-    SourceArgs S = solver_source_args(s);
-    S.lookahead = s->nbuf / 2;
-    if (s->has_source) BHR_CUDA_TRY(launch_source(S, 1, s->stream));
+    if (s->has_source) BHR_CUDA_TRY(launch_source(solver_source_args(s), 1, s->stream));
     if (int st = launch_stages(s, 0, false, false, e + 1)) return st;
     BHR_CUDA_TRY(launch_extract(solver_extract_args(s), s->stream));
     BHR_CUDA_TRY(cudaEventRecord(e[5], s->stream));
     s->steps_done++;
   }
   BHR_CUDA_TRY(cudaEventRecord(t1, s->stream));
+  if (s->has_source) BHR_CUDA_TRY(launch_first_sources(s));  // those of the steps that follow
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
   for (int i = 0; i < nsteps; i++)
     for (int j = s->has_source ? 0 : 1; j < 5; j++) {

@@ -57,9 +57,9 @@ typedef enum bhr_init_kind { BHR_INIT_ZERO = 0, BHR_INIT_GAUSSIAN = 1 } bhr_init
  * 128-thread block, four per SM; 64 x 8 tiles walked by two 256-thread
  * blocks per SM; stages 1 and 2 fused in one launch over 128-column strips
  * (the intermediate stage stays in shared memory; FP64 SSP-RK3 solves, stage
- * 3 as block8n).  Source-free FP64 SSP-RK3 solves whose grid fits one tile of
- * 64 columns x up to 32 rows per SM run resident (BHR_TILING_RESIDENT) where
- * the environment does not fix a tiling: up to 64 steps per launch, each
+ * 3 as block8n).  FP64 solves whose grid fits one tile of 64 columns x up to
+ * 16 rows per SM (source-free SSP-RK3: 32) run resident (BHR_TILING_RESIDENT)
+ * where the environment does not fix a tiling: up to 64 steps per launch, each
  * tile in its SM's shared memory. */
 typedef enum bhr_tiling {
   BHR_TILING_BLOCK8 = 0,

@@ -1,14 +1,14 @@
-"""Whole steps of small source-free grids in one cooperative launch: each
-tile stays on its SM, edges travel between neighbours stage by stage.
+"""Whole steps of small grids in one cooperative launch: each tile stays on
+its SM, edges travel between neighbours stage by stage.
 
 Against the oracle at the sizes where the tiling changes shape -- one strip
 (both radial ends in one tile), one tile per column of strips, tiles of 3, 8,
 9, 16, 17 and 32 rows (the limits of the kernel's three shapes on 148 SMs),
 segments of uneven height, the first grid that does not fit -- with even and
 odd m, the extraction column inside and at both ends, and step counts that
-leave launches of 1, 63, 64 and a remainder.  Tolerances are those of the
-other parity tests: fields 1e-12 of scale, waveform rows relative L2 1e-10,
-times bit-identical."""
+leave launches of 1, 63, 64 and a remainder.  With a source and with RK4
+against the stage launches.  Tolerances are those of the other parity tests:
+fields 1e-12 of scale, waveform rows relative L2 1e-10, times bit-identical."""
 import threading
 
 import numpy as np
@@ -73,13 +73,59 @@ def test_grids_that_do_not_fit_run_by_stage():
             assert s.info()["tiling"] != "resident"
 
 
-def test_a_trajectory_set_between_steps_leaves_the_resident_path():
-    """Source-free steps (one launch), then sourced ones (by stage), against
-    the oracle continued with the same state and a trajectory."""
-    N, M, a = 512, 32, 0.6
-    prm = bhr.Params(N=N, M=M, Xmin=-50.0, Xmax=50.0, a=a, m=2.0, dt=0.25 * 100.0 / N, T=60.0, Fr=5, out_start=0.0,
-                     ext_col=320, init_kind=bhr.BHR_INIT_GAUSSIAN, init_center=5.0, init_width=2.0)
-    rows = synthetic_plunge(a, prm.dt / 2.0, duration=prm.T)
+@pytest.mark.parametrize("N,M,src,rk4,kw", [
+    (64, 16, True, True, {}),       # 3-row tiles, one strip
+    (512, 32, True, False, {}),     # 3-row tiles
+    (896, 80, True, True, {}),      # 8-row tiles
+    (1024, 80, True, False, {}),    # 9-row tiles (two columns a thread)
+    (1024, 80, False, True, {}),
+    (1152, 128, True, False, {}),   # 16-row tiles, the tallest with a source and of RK4
+    (1152, 128, True, True, {}),
+    (9472, 16, False, True, {}),    # 148 strips
+    (512, 32, True, False, dict(PTSX=800, PTSY=3000)),  # two patch buffers: two steps a launch
+])
+def test_source_and_rk4_match_the_steps_by_stage(N, M, src, rk4, kw):
+    """A trajectory and RK4's four stages against the stage launches (which
+    the other parity tests hold to the oracle): a trajectory set after 70
+    steps, then launches of 1, 64 and fewer steps."""
+    T, dt = 60.0, 0.25 * min(100.0 / N, 1.5 * np.pi / M)
+    prm = bhr.Params(N=N, M=M, Xmin=-50.0, Xmax=50.0, a=0.6, m=2.0, dt=dt, T=T, Fr=5, out_start=0.0, ext_col=N * 5 // 8,
+                     integrator=bhr.BHR_RK4 if rk4 else bhr.BHR_SSPRK3, init_kind=bhr.BHR_INIT_GAUSSIAN,
+                     init_center=5.0, init_width=2.0, **kw)
+    rows = synthetic_plunge(prm.a, dt / 2.0, duration=T)
+    out, saved = [], None
+    for tiling in (None, "block8n", None):  # the third resumes the second's checkpoint
+        with pytest.MonkeyPatch.context() as mp:
+            if tiling:
+                mp.setenv("BHR_STAGE_TILING", tiling)
+            with bhr.Solver(prm) as s:
+                if len(out) < 2:
+                    s.step(70)
+                if src:
+                    s.set_trajectory(rows)
+                assert (s.info()["tiling"] == "resident") == (tiling is None)
+                if len(out) < 2:
+                    s.step(1)
+                    saved = s.checkpoint()
+                else:
+                    s.restore(saved)
+                for n in (66, 3):
+                    s.step(n)
+                out.append((s.get_state(), s.waveform(), s.get_extraction(), s.get_source()))
+    f1, w1, e1, s1 = out[1]
+    for f, w, e, so in (out[0], out[2]):
+        assert field_err(f, f1) <= FIELD_TOL and np.array_equal(w[0], w1[0])
+        assert np.linalg.norm(w[1] - w1[1]) <= WAVE_TOL * np.linalg.norm(w1[1])
+        assert np.linalg.norm(e[0] - e1[0]) <= WAVE_TOL * np.linalg.norm(e1[0])
+        assert all(np.array_equal(x, y) for x, y in zip(so, s1)) and (not src or np.max(np.abs(s1[0])) > 0)
+
+
+def test_a_source_on_taller_tiles_leaves_the_resident_path():
+    """Source-free steps (one launch), then sourced ones (by stage) on a grid
+    of 19-row tiles, against all steps by stage."""
+    prm = bhr.Params(N=2048, M=80, Xmin=-50.0, Xmax=50.0, a=0.6, m=2.0, dt=0.012, T=3.0, Fr=5, out_start=0.0,
+                     ext_col=1280, init_kind=bhr.BHR_INIT_GAUSSIAN, init_center=5.0, init_width=2.0)
+    rows = synthetic_plunge(prm.a, prm.dt / 2.0, duration=prm.T)
     out = []
     for tiling in (None, "block8n"):
         with pytest.MonkeyPatch.context() as mp:
