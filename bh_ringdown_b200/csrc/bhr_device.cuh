@@ -135,21 +135,29 @@ __device__ __forceinline__ double sqrt_nr(double x) {
 __device__ __forceinline__ double inv_bir(double b0, double b1, double s2) { return rcp_nr(fma(b1, s2, b0)); }
 
 // After a final stage has stored columns a0, a0 + 1 of RPT rows from b0 on:
-// psi at the recorded columns among them (read back by the thread that wrote
-// it, outside the row work, whose registers are all in use) to the history.
+// psi at the recorded column among them (never both) to the history, read back
+// by the thread that wrote it, outside the row work, whose registers are all
+// in use.  All loads come before the stores: the tile with the column ends the
+// stage, and a load and a store in turn took it 2 RPT trips to L2.
 template <int RPT>
 __device__ __forceinline__ void record_columns(double *hist, const int (&ext)[2], const RunState *rs, const int step,
                                                const double *out, const int N, const int M, const int a0,
                                                const int b0) {
   if (hist == nullptr) return;
+  const int e = ext[0] == a0 || ext[0] == a0 + 1 ? 0 : ext[1] == a0 || ext[1] == a0 + 1 ? 1 : -1;
+  if (e < 0) return;
+  double v[2][RPT];
 #pragma unroll
-  for (int e = 0; e < 2; e++) {
-    if (ext[e] != a0 && ext[e] != a0 + 1) continue;
-    double *h = hist + static_cast<size_t>(4 * ((rs->ks + step) % kHistSteps) + 2 * e) * M;
-    for (int b = max(b0, 3); b < min(b0 + RPT, M - 3); b++)
-      for (int pl = 0; pl < 2; pl++)
-        h[pl * M + b] = out[(static_cast<size_t>(pl) * M + b) * N + ext[e]];
-  }
+  for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+    for (int r = 0; r < RPT; r++)
+      if (b0 + r >= 3 && b0 + r < M - 3) v[pl][r] = out[(static_cast<size_t>(pl) * M + b0 + r) * N + ext[e]];
+  double *h = hist + static_cast<size_t>(4 * ((rs->ks + step) % kHistSteps) + 2 * e) * M + b0;
+#pragma unroll
+  for (int pl = 0; pl < 2; pl++)
+#pragma unroll
+    for (int r = 0; r < RPT; r++)
+      if (b0 + r >= 3 && b0 + r < M - 3) h[pl * M + r] = v[pl][r];
 }
 
 // Work item t of a launch group: the index of its solve in the group and

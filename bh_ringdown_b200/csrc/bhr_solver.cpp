@@ -48,12 +48,14 @@ static constexpr int kSequence = 16;
 static_assert(2 * kSequence <= kHistSteps, "the history holds two sequences");
 // A sequence is captured into a graph when at least kGraphSteps are left to
 // run, or the grid has fewer than kDirectPoints points.  A graph of 16 steps
-// costs 3.5 ms to capture, instantiate and destroy (4096 x 128 RK4, 600 steps:
-// 10 % of the solve) and frees the host of long runs; launched directly, a
-// step costs the host 10-15 us, which steps of small grids do not hide (us a
-// step, graph and direct: 2048 x 128 mixed 22.2 and 24.1, 1024 x 64 sourced 11.7
-// and 14.8, 4096 x 128 sourced 35.8 and 35.3).
-static constexpr int kGraphSteps = 4096;
+// costs 0.2 ms to capture, instantiate and destroy, and its launches follow
+// one another 0.3-1 us a step closer: it pays from 300-500 steps on (ms a
+// solve, direct and graph: 4096 x 128 of 100 steps 5.14 and 5.33, of 600 24.5
+// and 24.2, of 2000 78.8 and 77.2; 16384 x 128 of 600 69.3 and 68.9).
+// Launched directly, a step costs the host 10-15 us, which steps of small
+// grids do not hide (us a step, graph and direct: 2048 x 128 mixed 22.2 and
+// 24.1, 4096 x 128 sourced 35.8 and 35.3).
+static constexpr int kGraphSteps = 512;
 static constexpr size_t kDirectPoints = 400000;
 // Patch buffers of a solve take at most this much (two at least).
 static constexpr size_t kPatchBytes = 64u << 20;
