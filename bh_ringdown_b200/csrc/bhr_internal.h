@@ -90,6 +90,8 @@ struct StageArgs {
                         // input of the block this many places later in launch order (0: none,
                         // -1: stage_prefetch_ahead's default; launch_stage resolves it)
   int dir;              // narrow: the order the stage walks the grid's tiles in (StageDir)
+  int late;             // one-tile-per-block kernels: 1 where the next launch's blocks are let in as
+                        // this one's end (late_dependents)
   float *dout;          // mixed precision, stage 1: delta1 = dt L(u^n) in FP32, or nullptr
   double *zout;         // RK4 stage 2: z = (y1 + 2 y2 - u^n)/3, or nullptr
   int nbuf;             // source patch buffers
@@ -242,6 +244,7 @@ struct MixedArgs {
   double *hist;
   int ext[2];
   float dt, cx, cy, cyy, cko;
+  int late;             // as in StageArgs
 };
 struct MixedBatch {
   MixedMaps maps[2];    // stages 2 and 3

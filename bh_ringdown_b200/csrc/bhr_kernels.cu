@@ -509,7 +509,6 @@ __device__ __forceinline__ void stage_tile(const StageMaps &T, const StageArgs &
   if (tid == 0) tile_issue_setup<STAGE>(S, T, c0, b0);
   // Everything below reads what the earlier kernels of the step wrote.
   grid_dependency_wait();
-  launch_dependents();
   if (tid == 0) {
     tile_issue_state<STAGE>(S, T, c0, b0);
     tile_note_source(S, A);
@@ -519,6 +518,7 @@ __device__ __forceinline__ void stage_tile(const StageMaps &T, const StageArgs &
     if (kind == 1) tile_prefetch<STAGE>(*pm, pc0, pb0);
     if (kind == 2) tile_prefetch_next(*pm, pc0, pb0);
   }
+  if (!A.late) launch_dependents();  // else as the block ends
   const bool ok = mbar_wait_bounded(&S.bar, 0);
   if (!__syncthreads_and(ok)) {
     if (tid == 0) atomicCAS(A.err, 0, 5 /* BHR_TIMEOUT */);

@@ -122,7 +122,6 @@ __device__ __forceinline__ void mixed_tile(const MixedMaps &T, const MixedArgs &
     tma_load_2d(&S.rf[0][0], &T.rowf, b0, 0, &S.bar);
   }
   grid_dependency_wait();
-  launch_dependents();
   if (tid == 0) {
     tma_load_3d(&S.q[0][0][0], &T.q, c0 - 4, b0 - 3, 0, &S.bar);
     tma_load_3d(&S.p[0][0][0], &T.p, c0 - 4, b0, 2, &S.bar);
@@ -136,6 +135,7 @@ __device__ __forceinline__ void mixed_tile(const MixedMaps &T, const MixedArgs &
       if (STAGE == 3) tma_prefetch_3d(&pm->u1, pc0, pb0, 0);
     }
   }
+  if (!A.late) launch_dependents();  // else as the block ends
   const int a0 = c0 + 2 * tx;
   // The history of this thread's recorded column (the second of its two if
   // odd), written with the row: reading the column back after the rows held

@@ -163,6 +163,8 @@ double tortoise(double r, double a, double rpl, double rmn) {
 
 static int autotune_rows(bhr_solver *s);
 static bool runs_resident(const bhr_solver *s);
+static int late_dependents(int blocks, int next, int per_sm);
+static void history_columns(const bhr_solver *s, int ext[2]);
 static cudaError_t launch_first_sources(bhr_solver *s);
 
 extern "C" {
@@ -863,8 +865,22 @@ static int encode_maps(bhr_solver *s, int rows) {
 }
 
 
-// Stage tiling autotuner: per (device, N, M) the stage kernels are timed
-// on stages 1 and 2 (which write only the solve's scratch stages u1, u2):
+// The blocks of a stage launch, whether each has one tile, and how many an SM
+// holds; those of an FP32 stage (of stage 2 an SM holds four, but four are
+// hardly slower there than three: mixed 5120 x 64, 320 blocks, 22.9 us a step
+// let in at once, 23.4 spread).
+struct StageBlocks {
+  int stage, per_sm, mixed, mixed_per_sm = 3;
+  bool one_tile;
+  explicit StageBlocks(const bhr_solver *s)
+      : stage(s->p.N / TC * (s->p.M / s->tile_rows)),
+        per_sm(s->narrow ? 4 : 2),
+        mixed(s->p.N / TC * (s->p.M / kMixTileRows)),
+        one_tile(!s->persist && !s->ring && !s->strip12) {}
+};
+
+// Stage tiling autotuner: per (device, N, M, kind of step) the launches of
+// stages 1 and 2 (which write only the solve's scratch stages) are timed:
 // 8-row tiles on 128-thread blocks with the L2 prefetch one, two or four
 // SM-counts ahead or none (the staging depth), 8- and 16-row tiles one per
 // 256-thread block, the persistent 16-row kernels, the 8-row ring, and
@@ -872,14 +888,14 @@ static int encode_maps(bhr_solver *s, int rows) {
 // fastest is kept for the process.
 static int autotune_rows(bhr_solver *s) {
   static std::mutex mu;
-  // device, N, M, FP64 SSP-RK3, rows, persist, narrow, ring, strip12, ahead
+  // device, N, M, kind of step, rows, persist, narrow, ring, strip12, ahead
   static std::vector<std::array<int, 10>> cache;
   const bhr_params &p = s->p;
-  const int fused_ok = (!s->mixed && !s->rk4) ? 1 : 0;
+  const int kind = s->mixed ? 2 : s->rk4 ? 1 : 0;
   {
     std::lock_guard<std::mutex> lock(mu);
     for (auto &c : cache)
-      if (c[0] == p.device && c[1] == p.N && c[2] == p.M && c[3] == fused_ok) {
+      if (c[0] == p.device && c[1] == p.N && c[2] == p.M && c[3] == kind) {
         s->persist = c[5];
         s->narrow = c[6];
         s->ring = c[7];
@@ -894,15 +910,16 @@ static int autotune_rows(bhr_solver *s) {
   static const int cands[9][6] = {{8, 0, 1, 0, 0, 2}, {8, 0, 1, 0, 0, 1}, {8, 0, 1, 0, 0, 4}, {8, 0, 1, 0, 0, -1},
                                   {8, 0, 0, 0, 0, 2}, {16, 0, 0, 0, 0, 2}, {16, 1, 0, 0, 0, 0},
                                   {8, 0, 0, 1, 0, 0}, {8, 0, 1, 0, 1, 2}};
-  const int ncand = fused_ok ? 9 : 8;
+  const int ncand = kind == 0 ? 9 : 8;
   const int nsm = device_sm_count();
   double best_ms = 1e30;
   int best = 0;
   cudaEvent_t e0, e1;
   BHR_CUDA_TRY(cudaEventCreate(&e0));
   BHR_CUDA_TRY(cudaEventCreate(&e1));
-  // Stages 1 and 2 (they write only the solve's scratch stages u1, u2) of
-  // each candidate, or the fused launch that replaces them.
+  // Stages 1 and 2 (they write only the solve's scratch stages) of each
+  // candidate, or the fused launch that replaces them, and the launch that
+  // records a step of the tilings that do not record themselves.
   auto ahead_of = [&](int c) { return cands[c][5] < 0 ? 0 : cands[c][5] * nsm; };
   for (int c = 0; c < ncand; c++) {
     s->persist = cands[c][1];
@@ -913,6 +930,17 @@ static int autotune_rows(bhr_solver *s) {
     if (int st = encode_maps(s, cands[c][0])) return st;
     StageArgs A = solver_stage_args(s);
     A.src = nullptr;
+    const StageBlocks B(s);
+    MixedArgs X{};
+    if (s->mixed) {
+      X = solver_mixed_args(s);
+      X.e_out = s->e2f;
+      X.late = B.one_tile && late_dependents(B.mixed, B.stage, B.per_sm);
+      A.dout = s->d1f;
+    }
+    A.late = s->mixed ? late_dependents(B.stage, B.mixed, B.mixed_per_sm)
+                      : B.one_tile && late_dependents(B.stage, B.stage, B.per_sm);
+    history_columns(s, A.ext);
     for (int rep = 0; rep < 6; rep++) {
       if (rep == 2) BHR_CUDA_TRY(cudaEventRecord(e0, s->stream));
       if (s->strip12) {
@@ -922,8 +950,17 @@ static int autotune_rows(bhr_solver *s) {
       }
       A.vin = s->u0; A.un = s->u0; A.out = s->u1;
       BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
+      if (s->mixed) {
+        BHR_CUDA_TRY(launch_mixed_stage(2, s->mmaps[0], X, s->stream));
+        continue;
+      }
       A.vin = s->u1; A.un = s->u0; A.out = s->u2;
       BHR_CUDA_TRY(launch_stage(2, s->maps[1], A, s->stream));
+      if (s->persist || s->ring) {
+        A.hist = s->hist;
+        BHR_CUDA_TRY(launch_record(A, s->stream));
+        A.hist = nullptr;
+      }
     }
     BHR_CUDA_TRY(cudaEventRecord(e1, s->stream));
     BHR_CUDA_TRY(cudaEventSynchronize(e1));
@@ -938,7 +975,7 @@ static int autotune_rows(bhr_solver *s) {
   cudaEventDestroy(e1);
   {
     std::lock_guard<std::mutex> lock(mu);
-    cache.push_back({p.device, p.N, p.M, fused_ok, cands[best][0], cands[best][1], cands[best][2], cands[best][3],
+    cache.push_back({p.device, p.N, p.M, kind, cands[best][0], cands[best][1], cands[best][2], cands[best][3],
                      cands[best][4], ahead_of(best)});
   }
   s->persist = cands[best][1];
@@ -1062,6 +1099,21 @@ static void history_columns(const bhr_solver *s, int ext[2]) {
   ext[1] = a < 3 ? 4 : a >= N - 3 ? N - 5 : -1;
 }
 
+// Whether a launch of `blocks` lets the next launch's `next` blocks, of which
+// an SM holds `per_sm`, in only as its own end.  Let in at once they take the
+// slots in the order these free up, per_sm to the SMs that the first launch
+// leaves idle; in a launch of less than a wave that costs more than the
+// overlap gives wherever an even spread has fewer on an SM.  Where both
+// launches fit on different SMs there is nothing to spread.  us per step, at
+// once and as the blocks end: mixed 3072 x 64 20.7 and 17.8 (FP64 stage: 384
+// blocks, four an SM), 4096 x 64 21.7 and 18.9 (the FP32 stages: 256 of four
+// and three), RK4 3072 x 64 27.6 and 25.4; beyond, RK4 4096 x 64 28.6 and
+// 30.4 (512 blocks), mixed 5120 x 64 23.2 and 24.2 (320 blocks of three).
+static int late_dependents(int blocks, int next, int per_sm) {
+  const int sms = device_sm_count();
+  return next <= (per_sm - 1) * sms && blocks + next > sms;
+}
+
 // The stages of one step, the `step`-th of its sequence.  record: psi at the
 // history columns goes to the history.  flip: the step begins backward, where
 // stages turn.  `ev`: 4 events around the stages (the final one, and RK4's
@@ -1073,13 +1125,18 @@ static int launch_stages(bhr_solver *s, int step, bool record, bool flip, cudaEv
   // Consecutive stages walk the grid in opposite directions where the states
   // do not stay in L2 (kTurnBytes), so each starts on the tiles the one before
   // wrote last.
+  const StageBlocks B(s);
+  A.late = B.one_tile && late_dependents(B.stage, B.stage, B.per_sm);
   const bool turns = solver_turns(s);
   A.dir = !turns ? kSameWay : flip ? kBackward : kForward;
   auto turn = [&] {
     if (turns) A.dir = A.dir == kForward ? kBackward : kForward;
   };
   auto final_stage = [&](int stage, int map) -> cudaError_t {
-    if (!record) return launch_stage(stage, s->maps[map], A, s->stream);
+    if (!record) {  // the extraction follows
+      A.late = 0;
+      return launch_stage(stage, s->maps[map], A, s->stream);
+    }
     A.hist = s->hist;
     history_columns(s, A.ext);
     if (!s->persist && !s->ring) return launch_stage(stage, s->maps[map], A, s->stream);
@@ -1093,14 +1150,17 @@ static int launch_stages(bhr_solver *s, int step, bool record, bool flip, cudaEv
   if (s->mixed) {
     // u1 in FP64 and delta1 in FP32, then the FP32 stages 2 and 3.
     A.dout = s->d1f;
+    A.late = late_dependents(B.stage, B.mixed, B.mixed_per_sm);
     BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
     BHR_CUDA_TRY(mark(1));
     MixedArgs X = solver_mixed_args(s);
     X.e_out = s->e2f;
+    X.late = late_dependents(B.mixed, B.mixed, B.mixed_per_sm);
     BHR_CUDA_TRY(launch_mixed_stage(2, s->mmaps[0], X, s->stream));
     BHR_CUDA_TRY(mark(2));
     X.e_out = nullptr;
     X.u_out = s->u0;
+    X.late = record && B.one_tile && late_dependents(B.mixed, B.stage, B.per_sm);
     X.step = step;
     if (record) {
       X.hist = s->hist;
