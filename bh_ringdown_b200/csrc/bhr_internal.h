@@ -69,6 +69,10 @@ enum StageDir { kSameWay = 0, kForward = 1, kBackward = 2 };
 
 // Steps a solve's history holds: those of two sequences.
 constexpr int kHistSteps = 32;
+// Bytes of states (one solve's, or a batch's) from which on consecutive
+// stages walk the tiles in opposite directions.
+constexpr size_t kTurnBytes = 96u << 20;
+constexpr size_t kTurnMixedBytes = 128u << 20;  // the FP32 stages of mixed precision (of its FP64 states)
 
 struct StageArgs {
   const double *vin;    // stage input planes (also the TMA source)
@@ -254,9 +258,10 @@ using MixedGroup = WorkGroup<MixedArgs>;
 static_assert(sizeof(MixedGroup) + 64 <= 32764, "a kernel's parameters are limited to 32764 bytes");
 cudaError_t encode_mixed_maps(const float *in, const float *bbf, const float *colf, const float *rowf,
                               const double *u1, int N, int M, MixedMaps *maps);
-cudaError_t launch_mixed_stage(int stage, const MixedMaps &maps, const MixedArgs &a, cudaStream_t st);
+// backward: the tiles in reverse order.
+cudaError_t launch_mixed_stage(int stage, const MixedMaps &maps, const MixedArgs &a, bool backward, cudaStream_t st);
 // One launch of a mixed stage over a group of mixed solves (16-row tiles).
-cudaError_t launch_mixed_batch(int stage, const MixedBatch *solves, const MixedGroup &g, cudaStream_t st);
+cudaError_t launch_mixed_batch(int stage, const MixedBatch *solves, const MixedGroup &g, bool backward, cudaStream_t st);
 cudaError_t launch_to_float(const double *src, float *dst, size_t n, cudaStream_t st);
 // kc[4][M][N] (FP32): bb, ee, d_re, d_im formed in FP64 from the tables.
 cudaError_t launch_mixed_coef(const double *coltab, const double *rowtab, const double *bbt, float *kc, int N, int M,
@@ -312,8 +317,8 @@ constexpr int tiling_rows(int tiling) {
 constexpr int kMixTileRows = 16;
 // One launch of an FP64 stage over a group of a batch's solves (tiles of the
 // tiling's height).
-cudaError_t launch_stage_batch(int stage, int tiling, const BatchSolve *solves, const BatchGroup &g, int *err,
-                               cudaStream_t st);
+cudaError_t launch_stage_batch(int stage, int tiling, const BatchSolve *solves, const BatchGroup &g, bool backward,
+                               int *err, cudaStream_t st);
 cudaError_t launch_source_batch(const SourceArgs *args, int nsolves, int max_ptsy, int max_ptsx, cudaStream_t st);
 cudaError_t launch_extract_batch(const ExtractArgs *args, int nsolves, cudaStream_t st);
 cudaError_t launch_extract(const ExtractArgs &a, cudaStream_t st);

@@ -562,7 +562,7 @@ struct GridAhead {
 // Batch: the work item `n` places later in the group.  (Prefetching the
 // next stage's first items from the last blocks, as the single-solve
 // kernels do, measured no gain here.)
-template <int STAGE, int ROWS>
+template <int STAGE, int ROWS, bool BACK = false>
 struct GroupAhead {
   const BatchSolve *solves;
   const BatchGroup *G;
@@ -570,7 +570,7 @@ struct GroupAhead {
   __device__ __forceinline__ int operator()(const StageMaps *&pm, int &c0, int &b0) const {
     const int L = blockIdx.x + n;
     if (n <= 0 || L >= G->ntiles) return 0;
-    pm = &solves[G->solve[group_item(*G, L, ROWS, c0, b0)]].maps[STAGE - 1];
+    pm = &solves[G->solve[group_item(*G, BACK ? G->ntiles - 1 - L : L, ROWS, c0, b0)]].maps[STAGE - 1];
     return 1;
   }
 };
@@ -798,13 +798,14 @@ __global__ void __launch_bounds__(kRingThreads, kRingBlocksPerSM)
   stage_persistent<STAGE, kRingRows, kRingThreads, kRingBufs, false>(W, err);
 }
 
-template <int STAGE>
+// BACK: the group's work items in reverse order.
+template <int STAGE, bool BACK>
 __global__ void __launch_bounds__(kNarrowThreads, 4)
     stage_narrow_batch_kernel(const BatchSolve *solves, const __grid_constant__ BatchGroup G, int ahead) {
   int c0, b0;
-  const int i = group_item(G, blockIdx.x, 8, c0, b0);
+  const int i = group_item(G, BACK ? G.ntiles - 1 - static_cast<int>(blockIdx.x) : blockIdx.x, 8, c0, b0);
   stage_tile<STAGE, 8, kNarrowThreads>(solves[G.solve[i]].maps[STAGE - 1], G.args[i], c0, b0,
-                                       GroupAhead<STAGE, 8>{solves, &G, ahead});
+                                       GroupAhead<STAGE, 8, BACK>{solves, &G, ahead});
 }
 
 // ---- stages 1 and 2 fused over column strips (the strip12 tiling) --------
@@ -1574,7 +1575,8 @@ cudaError_t prepare_kernels() {
         if ((r = cudaFuncSetAttribute(stage_batch_kernel<S, 8>, kSmem, s8)) ||
             (r = cudaFuncSetAttribute(stage_batch_kernel<S, 16>, kSmem, s16)) ||
             (r = cudaFuncSetAttribute(stage_persistent_batch_kernel<S>, kSmem, sp)) ||
-            (r = cudaFuncSetAttribute(stage_narrow_batch_kernel<S>, kSmem, s8)) ||
+            (r = cudaFuncSetAttribute(stage_narrow_batch_kernel<S, false>, kSmem, s8)) ||
+            (r = cudaFuncSetAttribute(stage_narrow_batch_kernel<S, true>, kSmem, s8)) ||
             (r = cudaFuncSetAttribute(stage_ring_batch_kernel<S>, kSmem, sr)))
           return r;
       }
@@ -1585,8 +1587,8 @@ cudaError_t prepare_kernels() {
   return cudaSuccess;
 }
 
-cudaError_t launch_stage_batch(int stage, int tiling, const BatchSolve *solves, const BatchGroup &g, int *err,
-                               cudaStream_t st) {
+cudaError_t launch_stage_batch(int stage, int tiling, const BatchSolve *solves, const BatchGroup &g, bool backward,
+                               int *err, cudaStream_t st) {
   const int ntiles = g.ntiles;
   if (ntiles <= 0) return cudaSuccess;
   if (stage < 1 || stage > 3) return cudaErrorInvalidValue;
@@ -1600,8 +1602,9 @@ cudaError_t launch_stage_batch(int stage, int tiling, const BatchSolve *solves, 
         return launch_pdl(stage_ring_batch_kernel<S>, dim3(std::min(ntiles, kRingBlocksPerSM * sm_count())),
                           dim3(32, kRingThreads / 32), ring_smem_bytes(), st, solves, g, err);
       case kTilingBlock8n:
-        return launch_pdl(stage_narrow_batch_kernel<S>, dim3(ntiles), dim3(32, kNarrowThreads / 32),
-                          sizeof(StageSmem<8>) + 128, st, solves, g, stage_prefetch_ahead());
+        return launch_pdl(backward ? stage_narrow_batch_kernel<S, true> : stage_narrow_batch_kernel<S, false>,
+                          dim3(ntiles), dim3(32, kNarrowThreads / 32), sizeof(StageSmem<8>) + 128, st, solves, g,
+                          stage_prefetch_ahead());
       case kTilingBlock8:
         return launch_pdl(stage_batch_kernel<S, 8>, dim3(ntiles), dim3(32, STAGE_THREADS / 32),
                           sizeof(StageSmem<8>) + 128, st, solves, g, stage_prefetch_ahead());

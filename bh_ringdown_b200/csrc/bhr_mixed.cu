@@ -68,13 +68,16 @@ __device__ __forceinline__ float ko8f(const float *v, int c) {
 }
 
 // Single solve: the tile `n` places after this block's in launch order
-// (n = 0: none).
+// (n = 0: none).  BACK: the order is from the last tile to the first.
+template <bool BACK>
 struct MixGridAhead {
   const MixedMaps *T;
   int n;
   __device__ __forceinline__ bool operator()(const MixedMaps *&pm, int &c0, int &b0) const {
-    const int L = blockIdx.y * gridDim.x + blockIdx.x + n;
-    if (n <= 0 || L >= static_cast<int>(gridDim.x * gridDim.y)) return false;
+    const int ntiles = static_cast<int>(gridDim.x * gridDim.y);
+    int L = blockIdx.y * gridDim.x + blockIdx.x + n;
+    if (n <= 0 || L >= ntiles) return false;
+    if (BACK) L = ntiles - 1 - L;
     pm = T;
     c0 = (L % gridDim.x) * TC;
     b0 = (L / gridDim.x) * kMixRows;
@@ -82,7 +85,7 @@ struct MixGridAhead {
   }
 };
 // Batch: the work item `n` places later in the launch group.
-template <int STAGE>
+template <int STAGE, bool BACK>
 struct MixGroupAhead {
   const MixedBatch *solves;
   const MixedGroup *G;
@@ -90,14 +93,14 @@ struct MixGroupAhead {
   __device__ __forceinline__ bool operator()(const MixedMaps *&pm, int &c0, int &b0) const {
     const int L = blockIdx.x + n;
     if (n <= 0 || L >= G->ntiles) return false;
-    pm = &solves[G->solve[group_item(*G, L, kMixRows, c0, b0)]].maps[STAGE - 2];
+    pm = &solves[G->solve[group_item(*G, BACK ? G->ntiles - 1 - L : L, kMixRows, c0, b0)]].maps[STAGE - 2];
     return true;
   }
 };
 // One 64 x 16 tile (columns c0.., rows b0..) of stage 2 or 3.  Thread 0
 // prefetches into L2 the input of the later tile `ahead` names, so that the
 // block which takes it finds its loads there.
-template <int STAGE, class Ahead>
+template <int STAGE, bool RECORD, class Ahead>
 __device__ __forceinline__ void mixed_tile(const MixedMaps &T, const MixedArgs &A, const int c0, const int b0,
                                            const Ahead ahead) {
   constexpr int ROWS = kMixRows, RPT = ROWS / (kMixThreads / 32);
@@ -140,7 +143,7 @@ __device__ __forceinline__ void mixed_tile(const MixedMaps &T, const MixedArgs &
   // The history of this thread's recorded column (the second of its two if
   // odd), written with the row: reading the column back after the rows held
   // the step up by 0.7 us (4096 x 128, 31.0 -> 30.3).
-  const int e = STAGE < 3 || A.hist == nullptr ? -1 : (A.ext[0] & ~1) == a0 ? 0 : (A.ext[1] & ~1) == a0 ? 1 : -1;
+  const int e = !RECORD || A.hist == nullptr ? -1 : (A.ext[0] & ~1) == a0 ? 0 : (A.ext[1] & ~1) == a0 ? 1 : -1;
   const bool odd = e >= 0 && (A.ext[e] & 1);
   double *const h = e < 0 ? nullptr : A.hist + static_cast<size_t>(4 * ((A.rs->ks + A.step) % kHistSteps) + 2 * e) * M;
   const bool ok = mbar_wait_bounded(&S.bar, 0);
@@ -339,21 +342,22 @@ __device__ __forceinline__ void mixed_tile(const MixedMaps &T, const MixedArgs &
   else rows(std::false_type{});
 }
 
-template <int STAGE>
+template <int STAGE, bool BACK>
 __global__ void __launch_bounds__(kMixThreads, mix_blocks_per_sm<STAGE>())
     mixed_stage_kernel(const __grid_constant__ MixedMaps T, const MixedArgs A, int ahead) {
-  mixed_tile<STAGE>(T, A, blockIdx.x * TC, blockIdx.y * kMixRows, MixGridAhead{&T, ahead});
+  const int cx = BACK ? gridDim.x - 1 - blockIdx.x : blockIdx.x, cy = BACK ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
+  mixed_tile<STAGE, STAGE == 3>(T, A, cx * TC, cy * kMixRows, MixGridAhead<BACK>{&T, ahead});
 }
 
 // Mixed-precision solves of a batch: block -> (solve, tile), work item
 // blockIdx.x of the launch group (its `solve` entries index the MixedBatch
 // array).
-template <int STAGE>
+template <int STAGE, bool BACK>
 __global__ void __launch_bounds__(kMixThreads, mix_blocks_per_sm<STAGE>())
     mixed_batch_kernel(const MixedBatch *solves, const __grid_constant__ MixedGroup G, int ahead) {
   int c0, b0;
-  const int i = group_item(G, blockIdx.x, kMixRows, c0, b0);
-  mixed_tile<STAGE>(solves[G.solve[i]].maps[STAGE - 2], G.args[i], c0, b0, MixGroupAhead<STAGE>{solves, &G, ahead});
+  const int i = group_item(G, BACK ? G.ntiles - 1 - static_cast<int>(blockIdx.x) : blockIdx.x, kMixRows, c0, b0);
+  mixed_tile<STAGE, false>(solves[G.solve[i]].maps[STAGE - 2], G.args[i], c0, b0, MixGroupAhead<STAGE, BACK>{solves, &G, ahead});
 }
 
 // bb, ee = Ataurho + bb, d_re = (Brho_re - bb Btau_re) - bb' ee and
@@ -443,27 +447,38 @@ cudaError_t encode_mixed_maps(const float *in, const float *bbf, const float *co
 cudaError_t prepare_mixed_kernels() {
   cudaError_t e;
   const int s2 = static_cast<int>(mix_smem_bytes<2>()), s3 = static_cast<int>(mix_smem_bytes<3>());
-  if ((e = cudaFuncSetAttribute(mixed_stage_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2)) ||
-      (e = cudaFuncSetAttribute(mixed_stage_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3)) ||
-      (e = cudaFuncSetAttribute(mixed_batch_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2)) ||
-      (e = cudaFuncSetAttribute(mixed_batch_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, s3)))
+  constexpr auto kSmem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if ((e = cudaFuncSetAttribute(mixed_stage_kernel<2, false>, kSmem, s2)) ||
+      (e = cudaFuncSetAttribute(mixed_stage_kernel<2, true>, kSmem, s2)) ||
+      (e = cudaFuncSetAttribute(mixed_stage_kernel<3, false>, kSmem, s3)) ||
+      (e = cudaFuncSetAttribute(mixed_stage_kernel<3, true>, kSmem, s3)) ||
+      (e = cudaFuncSetAttribute(mixed_batch_kernel<2, false>, kSmem, s2)) ||
+      (e = cudaFuncSetAttribute(mixed_batch_kernel<2, true>, kSmem, s2)) ||
+      (e = cudaFuncSetAttribute(mixed_batch_kernel<3, false>, kSmem, s3)) ||
+      (e = cudaFuncSetAttribute(mixed_batch_kernel<3, true>, kSmem, s3)))
     return e;
   return cudaSuccess;
 }
 
-cudaError_t launch_mixed_stage(int stage, const MixedMaps &maps, const MixedArgs &a, cudaStream_t st) {
+cudaError_t launch_mixed_stage(int stage, const MixedMaps &maps, const MixedArgs &a, bool backward, cudaStream_t st) {
   const dim3 grid(a.N / TC, a.M / kMixRows), block(32, kMixThreads / 32);
   const int ahead = stage_prefetch_ahead();
-  if (stage == 2) return launch_pdl(mixed_stage_kernel<2>, grid, block, mix_smem_bytes<2>(), st, maps, a, ahead);
-  return launch_pdl(mixed_stage_kernel<3>, grid, block, mix_smem_bytes<3>(), st, maps, a, ahead);
+  if (stage == 2)
+    return launch_pdl(backward ? mixed_stage_kernel<2, true> : mixed_stage_kernel<2, false>, grid, block,
+                      mix_smem_bytes<2>(), st, maps, a, ahead);
+  return launch_pdl(backward ? mixed_stage_kernel<3, true> : mixed_stage_kernel<3, false>, grid, block,
+                    mix_smem_bytes<3>(), st, maps, a, ahead);
 }
 
-cudaError_t launch_mixed_batch(int stage, const MixedBatch *solves, const MixedGroup &g, cudaStream_t st) {
+cudaError_t launch_mixed_batch(int stage, const MixedBatch *solves, const MixedGroup &g, bool backward, cudaStream_t st) {
   if (g.ntiles <= 0) return cudaSuccess;
   const dim3 grid(g.ntiles), block(32, kMixThreads / 32);
   const int ahead = stage_prefetch_ahead();
-  if (stage == 2) return launch_pdl(mixed_batch_kernel<2>, grid, block, mix_smem_bytes<2>(), st, solves, g, ahead);
-  return launch_pdl(mixed_batch_kernel<3>, grid, block, mix_smem_bytes<3>(), st, solves, g, ahead);
+  if (stage == 2)
+    return launch_pdl(backward ? mixed_batch_kernel<2, true> : mixed_batch_kernel<2, false>, grid, block,
+                      mix_smem_bytes<2>(), st, solves, g, ahead);
+  return launch_pdl(backward ? mixed_batch_kernel<3, true> : mixed_batch_kernel<3, false>, grid, block,
+                    mix_smem_bytes<3>(), st, solves, g, ahead);
 }
 
 cudaError_t launch_mixed_coef(const double *coltab, const double *rowtab, const double *bbt, float *kc, int N, int M,

@@ -951,7 +951,7 @@ static int autotune_rows(bhr_solver *s) {
       A.vin = s->u0; A.un = s->u0; A.out = s->u1;
       BHR_CUDA_TRY(launch_stage(1, s->maps[0], A, s->stream));
       if (s->mixed) {
-        BHR_CUDA_TRY(launch_mixed_stage(2, s->mmaps[0], X, s->stream));
+        BHR_CUDA_TRY(launch_mixed_stage(2, s->mmaps[0], X, false, s->stream));
         continue;
       }
       A.vin = s->u1; A.un = s->u0; A.out = s->u2;
@@ -1081,15 +1081,18 @@ ExtractArgs bhr::solver_extract_args(bhr_solver *s) {
   return E;
 }
 
-// Solves whose states take this much and more are walked back and forth.
+// Solves whose states take kTurnBytes and more are walked back and forth.
 // Measured (us per step, same way -> in turn): 8192 x 128 63.0 -> 62.2 (100 MB
 // of states), 16000 x 256 201 -> 197, 16384 x 256 plunge 204 -> 200; below,
 // where L2 holds the states in any order, nothing is gained and the last
-// blocks' prefetch of the next stage's first tiles would be lost.
-static constexpr size_t kTurnBytes = 96u << 20;
-static bool solver_turns(const bhr_solver *s) {
-  return s->narrow && !s->strip12 && (s->rk4 ? 4 : 3) * sizeof(double) * 4 * static_cast<size_t>(s->p.N) * s->p.M >= kTurnBytes;
+// blocks' prefetch of the next stage's first tiles would be lost.  Mixed
+// precision: the FP64 stage begins forward and backward from step to step
+// (8192 x 128 53.4 -> 52.5, 8192 x 160 63.9 -> 62.5), the FP32 stages turn with
+// it from kTurnMixedBytes on (8192 x 128 53.4 with them, 8192 x 192 73.0 -> 70.9).
+static size_t state_bytes(const bhr_solver *s) {
+  return (s->rk4 ? 4 : 3) * sizeof(double) * 4 * static_cast<size_t>(s->p.N) * s->p.M;
 }
+static bool solver_turns(const bhr_solver *s) { return s->narrow && !s->strip12 && state_bytes(s) >= kTurnBytes; }
 
 // The columns a step's history keeps: the extraction column, or the two
 // interior ones its closure is made of.
@@ -1156,7 +1159,8 @@ static int launch_stages(bhr_solver *s, int step, bool record, bool flip, cudaEv
     MixedArgs X = solver_mixed_args(s);
     X.e_out = s->e2f;
     X.late = late_dependents(B.mixed, B.mixed, B.mixed_per_sm);
-    BHR_CUDA_TRY(launch_mixed_stage(2, s->mmaps[0], X, s->stream));
+    const bool turn32 = turns && state_bytes(s) >= kTurnMixedBytes;
+    BHR_CUDA_TRY(launch_mixed_stage(2, s->mmaps[0], X, turn32 && !flip, s->stream));
     BHR_CUDA_TRY(mark(2));
     X.e_out = nullptr;
     X.u_out = s->u0;
@@ -1166,7 +1170,7 @@ static int launch_stages(bhr_solver *s, int step, bool record, bool flip, cudaEv
       X.hist = s->hist;
       history_columns(s, X.ext);
     }
-    BHR_CUDA_TRY(launch_mixed_stage(3, s->mmaps[1], X, s->stream));
+    BHR_CUDA_TRY(launch_mixed_stage(3, s->mmaps[1], X, turn32 && flip, s->stream));
   } else if (s->rk4) {
     // Classical RK4, the step's source held fixed in all four stages:
     // y1 = u + dt/2 L(u); y2 = u + dt/2 L(y1), z = (y1 + 2 y2 - u)/3;
