@@ -71,6 +71,20 @@ def env_rank():
             int(os.environ.get("WORLD_SIZE", 1)))
 
 
+def gpu_launches(steps, one_by_one, with_source):
+    """Kernels the timed region launches.  A step has three stages (RK4: four).
+    Steps timed alone: the extraction of each, and one launch of the sources of
+    16 steps every 16.  Steps back to back, per sequence of up to 16: the step
+    clock, the sources of 16 steps, and the two extraction kernels of the
+    sequence before, which the last sequence's follow."""
+    stages = steps * (4 if INTEGRATOR == "rk4" else 3)
+    sequences = -(-steps // 16)
+    source = sequences if with_source else 0
+    if one_by_one:
+        return stages + steps + source
+    return stages + sequences + source + 2 * (sequences + 1)
+
+
 def measured_peak():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     try:
@@ -370,11 +384,9 @@ def run_ours(args, rank, local_rank, world):
                           "stage3+4" if INTEGRATOR == "rk4" else "stage3": per_kernel[3] / nprof,
                           "extract": per_kernel[4] / nprof,
                           "note": "breakdown only: eager launches each timed alone (no programmatic overlap "
-                                  "between kernels); source and extract run on a side stream beside stages 1 "
-                                  "and 2, timed from the side stream's fork to the kernel's end"},
-            # per step: the stages, the step-clock kernel, the extraction (of the
-            # previous step, beside stage 2) and the source when there is one
-            "gpu_launches": args.steps * ((6 if with_source else 5) + (1 if INTEGRATOR == "rk4" else 0)),
+                                  "between kernels); in the timed steps source and extraction run once per "
+                                  "sequence of up to 16 steps, beside the stages"},
+            "gpu_launches": gpu_launches(args.steps, resident, with_source),
             "e2e": e2e,
             "clocks": clocks,
             "cpu_baseline": cpu,

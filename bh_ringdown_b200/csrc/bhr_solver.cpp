@@ -57,6 +57,10 @@ static_assert(2 * kSequence <= kHistSteps, "the history holds two sequences");
 // 24.1, 4096 x 128 sourced 35.8 and 35.3).
 static constexpr int kGraphSteps = 512;
 static constexpr size_t kDirectPoints = 400000;
+// Calls of up to this many steps run them one by one: a sequence's fork, clock
+// and extraction are 14 us (8192 x 128, wall us of two steps: 141 one by one, 158
+// as a sequence; of four 269 and 279, of five 345 and 337).
+static constexpr int kFewSteps = 4;
 // Patch buffers of a solve take at most this much (two at least).
 static constexpr size_t kPatchBytes = 64u << 20;
 
@@ -165,7 +169,7 @@ static int autotune_rows(bhr_solver *s);
 static bool runs_resident(const bhr_solver *s);
 static int late_dependents(int blocks, int next, int per_sm);
 static void history_columns(const bhr_solver *s, int ext[2]);
-static cudaError_t launch_first_sources(bhr_solver *s);
+static cudaError_t launch_sources_ahead(bhr_solver *s, int done);
 
 extern "C" {
 
@@ -804,7 +808,8 @@ int bhr_solver_set_trajectory(bhr_solver *s, const double *rows, int nrows) {
     }
   }
   // The patches of the first sequence (later ones are built beside the stages).
-  BHR_CUDA_TRY(launch_first_sources(s));
+  s->built = 0;
+  if (!runs_resident(s)) BHR_CUDA_TRY(launch_sources_ahead(s, s->steps_done));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
   // The launch arguments now carry the source and the new records: step
   // graphs captured before (steps taken without a trajectory) are rebuilt.
@@ -1218,11 +1223,15 @@ static bool runs_resident(const bhr_solver *s) {
   return s->resident && (!s->has_source || s->rgeom.rmax <= kResidentSourceRows);
 }
 
-// The patches of a sequence from the current step on, before the first.
-// (A resident solve builds those of a launch ahead of it.)
-static cudaError_t launch_first_sources(bhr_solver *s) {
-  if (runs_resident(s)) return cudaSuccess;
-  return launch_source(solver_source_args(s), s->nbuf / 2, s->stream);
+// The patches of the steps from done on that are not there yet, up to a
+// sequence's (resident launches build their own).
+static cudaError_t launch_sources_ahead(bhr_solver *s, int done) {
+  const int from = std::max(s->built, done), to = done + s->nbuf / 2;
+  if (from >= to) return cudaSuccess;
+  SourceArgs S = solver_source_args(s);
+  S.lookahead = from - done;
+  s->built = to;
+  return launch_source(S, to - from, s->stream);
 }
 
 // The extraction of the steps done and not yet extracted (kSequence at most).
@@ -1243,14 +1252,15 @@ static cudaError_t launch_extraction(bhr_solver *s, cudaStream_t st) {
 // another directly, each overlapping the tail of the one before; with the
 // fork and join inside every step (and a clock launch and an extraction per
 // step) a step took 2-4 us more: 8192 x 128 62.3 -> 59.5, 4096 x 128 35.3 -> 33.5.
-// A single step extracts itself and then builds its one source.
+// A single step is extracted after its stages and builds no sources
+// (enqueue_steps has those of nbuf / 2 steps built at a time): a side stream
+// beside a single step costs more than it hides (8192 x 128 sourced, device us
+// a step: 72.3 with source and extraction beside the stages, 69.7 like this).
 static int launch_sequence(bhr_solver *s, int count) {
   SourceArgs S = solver_source_args(s);
   if (count == 1) {
     if (int st = launch_stages(s, 0, false, false)) return st;
     BHR_CUDA_TRY(launch_extract(solver_extract_args(s), s->stream));
-    S.lookahead = s->nbuf / 2 - 1;  // the clock has been advanced
-    if (s->has_source) BHR_CUDA_TRY(launch_source(S, 1, s->stream));
     return BHR_OK;
   }
   BHR_CUDA_TRY(cudaEventRecord(s->fork, s->stream));
@@ -1369,11 +1379,20 @@ static int enqueue_resident(bhr_solver *s, int nsteps, int *done) {
   return BHR_OK;
 }
 
-// The graphs a call of nsteps by stage will use: of one step for calls of one
-// step, of a full sequence for long runs.
+// A single step of a resident solve goes by stage as well (three at most where
+// a tile has more than 16 rows): a resident launch loads and stores the whole
+// grid and has two extraction launches behind it.  Wall us a call, by stage and
+// resident: 1024 x 64, one step 26.7 and 33.7, two 40 and 39; 2048 x 128, one
+// 39 and 50, two 65 and 75, three 91 and 98, four 116 and 114.
+static bool call_is_resident(const bhr_solver *s, int nsteps) {
+  return nsteps > (s->rgeom.rmax > kResidentSourceRows ? 3 : 1) && runs_resident(s);
+}
+
+// The graphs a call of nsteps by stage will use: of one step for calls of few
+// steps, of a full sequence for long runs.
 static int prepare_graphs(bhr_solver *s, int nsteps) {
-  if (runs_resident(s)) return BHR_OK;
-  if (nsteps == 1 && !s->g1) return capture_sequence(s, 1, &s->g1);
+  if (call_is_resident(s, nsteps)) return BHR_OK;
+  if (nsteps <= kFewSteps && !s->g1) return capture_sequence(s, 1, &s->g1);
   const int length = sequence_length(s);
   const bool graph = s->nt - s->steps_done >= kGraphSteps || static_cast<size_t>(s->p.N) * s->p.M < kDirectPoints;
   if (length > 1 && nsteps >= length && graph && !s->gb)
@@ -1383,26 +1402,30 @@ static int prepare_graphs(bhr_solver *s, int nsteps) {
 
 static int enqueue_steps(bhr_solver *s, int nsteps) {
   if (nsteps <= 0) return BHR_OK;
-  if (runs_resident(s)) {
+  if (call_is_resident(s, nsteps)) {
     int done = 0;
+    s->built = 0;
     if (int st = enqueue_resident(s, nsteps, &done)) return st;
     nsteps -= done;
     if (nsteps <= 0) return BHR_OK;
-    if (s->has_source) BHR_CUDA_TRY(launch_first_sources(s));
   }
   if (int st = prepare_graphs(s, nsteps)) return st;
-  const int length = sequence_length(s);
+  const int length = nsteps <= kFewSteps ? 1 : sequence_length(s);
   bool pending = false;  // a sequence has run and is not extracted
   for (int left = nsteps; left > 0;) {
-    const int n = std::min(left, length);
+    const int n = std::min(left, length), done = s->steps_done + nsteps - left;
+    if (s->has_source && (n > 1 || s->built <= done)) BHR_CUDA_TRY(launch_sources_ahead(s, done));
     if (n == 1 && pending) {
       BHR_CUDA_TRY(launch_extraction(s, s->stream));
       pending = false;
     }
-    if (n > 1) pending = true;
+    if (n > 1) {
+      pending = true;
+      s->built += n;
+    }
     if (n == 1 && s->g1) {
       BHR_CUDA_TRY(cudaGraphLaunch(s->g1, s->stream));
-    } else if (n == length && s->gb) {
+    } else if (n > 1 && n == length && s->gb) {
       BHR_CUDA_TRY(cudaGraphLaunch(s->gb, s->stream));
     } else if (int st = launch_sequence(s, n)) {
       return st;
@@ -1692,7 +1715,8 @@ int bhr_solver_restore(bhr_solver *s, const void *buf, size_t size) {
   }
   BHR_CUDA_TRY(cudaMemcpyAsync(s->rs, &h.rs, sizeof(RunState), cudaMemcpyHostToDevice, s->stream));
   // The patches of the sequence the solve resumes with.
-  if (s->has_source) BHR_CUDA_TRY(launch_first_sources(s));
+  s->built = 0;
+  if (s->has_source && !runs_resident(s)) BHR_CUDA_TRY(launch_sources_ahead(s, h.steps_done));
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
   s->steps_done = h.steps_done;
   return BHR_OK;
@@ -1758,7 +1782,7 @@ int bhr_solver_profile(bhr_solver *s, int nsteps, double *avg_ms5, double *total
     s->steps_done++;
   }
   BHR_CUDA_TRY(cudaEventRecord(t1, s->stream));
-  if (s->has_source) BHR_CUDA_TRY(launch_first_sources(s));  // those of the steps that follow
+  s->built = 0;
   BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
   for (int i = 0; i < nsteps; i++)
     for (int j = s->has_source ? 0 : 1; j < 5; j++) {

@@ -60,6 +60,7 @@ struct bhr_solver {
   unsigned long long rseq = 1;   // number of the next launch's first edge words
   int steps_done = 0;
   int nbuf = 2;        // source patch buffers
+  int built = 0;       // the patches of the steps up to this one, from steps_done on, are there (by stage)
   // Captured graphs: one step, and a full sequence of steps.
   cudaGraphExec_t g1 = nullptr, gb = nullptr;
   // Per-step source records past the first chunk are built and uploaded by

@@ -57,3 +57,36 @@ def test_any_split_of_a_run_gives_the_same_fields(tiling, kw, monkeypatch):
         for a, b in zip(list(p0) + list(e0), list(p) + list(e)):
             assert np.linalg.norm(a - b) <= 1e-13 * np.linalg.norm(a)
         assert all(np.array_equal(a, b) for a, b in zip(s0, so))
+
+
+@pytest.mark.parametrize("N,M,src", [(256, 32, True), (256, 32, False), (2048, 96, False), (6400, 64, True)])
+def test_host_reads_see_a_single_steps_extraction(N, M, src):
+    """A single step is extracted beside the next step, or by the first read
+    that needs it: whatever is read after each of seven single steps (then a
+    longer call, and single steps again) is what a run without reads has, on
+    grids that run resident and by stage."""
+    dt = 0.25 * min(100.0 / N, 1.6 * np.pi / M)
+    prm = bhr.Params(N=N, M=M, Xmin=-50.0, Xmax=50.0, a=0.6, m=2.0, dt=dt, T=100.0 * dt, Fr=2, out_start=0.0,
+                     ext_col=N * 6 // 10, init_kind=bhr.BHR_INIT_GAUSSIAN, init_center=10.0)
+    rows = synthetic_plunge(prm.a, dt / 2.0, duration=prm.T)
+    readers = [lambda s: s.info()["rows_done"], lambda s: s.waveform(), lambda s: s.psi_samples(),
+               lambda s: s.get_extraction(), lambda s: s.get_state(), lambda s: s.checkpoint(),
+               lambda s: s.set_state(*s.get_state())]
+    out = []
+    for read in (True, False):
+        with bhr.Solver(prm) as s:
+            if src:
+                s.set_trajectory(rows)
+            for k in range(7):
+                s.step(1)
+                if read:
+                    readers[k](s)
+                    assert s.info()["rows_done"] == len(s.waveform()[0]) == k // 2 + 1
+            for n in (20, 1, 1, 17, 1):
+                s.step(n)
+            assert s.info()["rows_done"] == 24
+            out.append((s.get_state(), s.waveform(), s.psi_samples(), s.get_extraction()))
+    (f0, w0, p0, e0), (f1, w1, p1, e1) = out
+    assert all(np.array_equal(a, b) for a, b in zip(f0, f1)) and np.array_equal(w0[0], w1[0])
+    for a, b in zip([w0[1], *p0, *e0], [w1[1], *p1, *e1]):
+        assert np.linalg.norm(a - b) <= 1e-13 * np.linalg.norm(b)
