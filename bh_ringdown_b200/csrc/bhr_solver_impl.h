@@ -52,8 +52,8 @@ struct bhr_solver {
   int ring = 0;        // 1: 8-row tiles through 2-buffer rings, two 256-thread blocks per SM
   int strip12 = 0;     // 1: stages 1 and 2 in one launch over column strips (FP64 SSP-RK3; stage 3 block8n)
   bhr::StripMaps smaps;
-  // Source-free FP64 SSP-RK3 steps of a small grid: several steps per
-  // cooperative launch (bhr_resident.cu) instead of stage launches.
+  // FP64 steps of a small grid: several steps per cooperative launch
+  // (bhr_resident.cu) instead of stage launches.
   bool resident = false;
   bhr::ResidentGeom rgeom{};
   ulonglong2 *inbox = nullptr;   // edge words of the blocks
