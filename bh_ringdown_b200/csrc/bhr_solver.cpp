@@ -52,9 +52,9 @@ static_assert(2 * kSequence <= kHistSteps, "the history holds two sequences");
 // one another 0.3-1 us a step closer: it pays from 300-500 steps on (ms a
 // solve, direct and graph: 4096 x 128 of 100 steps 5.14 and 5.33, of 600 24.5
 // and 24.2, of 2000 78.8 and 77.2; 16384 x 128 of 600 69.3 and 68.9).
-// Launched directly, a step costs the host 10-15 us, which steps of small
-// grids do not hide (us a step, graph and direct: 2048 x 128 mixed 22.2 and
-// 24.1, 4096 x 128 sourced 35.8 and 35.3).
+// Launched directly, a step costs the host 10 us and more, which steps of small
+// grids hide on a fast host only (us a step, graph and direct: 1024 x 64 mixed
+// 12.5 and 13.3, 2048 x 128 mixed 19.1 and 20.0, 4096 x 128 sourced 34.3 and 35.2).
 static constexpr int kGraphSteps = 512;
 static constexpr size_t kDirectPoints = 400000;
 // Calls of up to this many steps run them one by one: a sequence's fork, clock
