@@ -16,18 +16,18 @@
 // after that: q's edges travel while p is formed, p's while the next q is.
 //
 // Measured on 148 SMs, us per step (three stages), stage launches -> here:
-// 256 x 32 10.4 -> 5.2, 1024 x 64 12.7 -> 6.2, 2048 x 64 14.8 -> 10.0,
-// 2048 x 96 21.0 -> 19.1, 2048 x 128 23.2 -> 21.6, 4096 x 64 22.7 -> 20.8.
+// 256 x 32 10.4 -> 5.0, 1024 x 64 12.7 -> 5.8, 2048 x 64 14.8 -> 9.6,
+// 2048 x 96 21.0 -> 19.0, 2048 x 128 23.2 -> 21.3, 4096 x 64 22.7 -> 20.7.
 // With a source (the patches of a launch's steps are built before it: 0.5 us a
-// step) 512 x 32 13.1 -> 5.8, 1024 x 64 11.7 -> 6.8, 2048 x 64 15.2 -> 10.7;
-// RK4 512 x 32 14.0 -> 6.7, 1024 x 64 15.1 -> 7.9, 1536 x 64 20.1 -> 11.0.
+// step) 512 x 32 13.1 -> 5.5, 1024 x 64 11.7 -> 6.4, 2048 x 64 15.2 -> 10.4;
+// RK4 512 x 32 14.0 -> 6.7, 1024 x 64 15.1 -> 7.4, 1536 x 64 20.1 -> 11.0.
 // Taller tiles with a source lose to the stage launches, which build sources
-// beside the stages (2048 x 128 22.5 there, 23.7 here; 1152 x 256 23.2, 24.1),
+// beside the stages (2048 x 128 22.2 there, 23.7 here; 1152 x 256 23.2, 24.1),
 // and RK4's z takes their shared memory: both stop at 16 rows.
-// At 1024 x 64 (7-row tiles) 4.5 us of the 6.2 are a lone row's instruction
-// stream (latency of FP64 and shared-memory chains with 3-4 warps a
-// scheduler), 1.4 us waiting for edges; from 9 rows on the FP64 issue rate
-// counts, and taller tiles than 32 rows do not fit.
+// At 1024 x 64 (7-row tiles) about three quarters of the step are a lone row's
+// instruction stream (latency of FP64 and shared-memory chains with 4 warps a
+// scheduler), the rest waiting for edges; from 9 rows on the FP64 issue rate counts, and
+// taller tiles than 32 rows do not fit.
 //
 // The extraction column of every step goes to a history buffer, which
 // chunk_integrate_kernel and chunk_project_kernel turn into the time
@@ -292,6 +292,17 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
       for (int f = 0; f < CF_TILE; f++) get<COLS>(cf[f], A.coltab + static_cast<size_t>(f) * N + a0);
       row_coef<COLS>(C, A, w, cf, A.rowtab[static_cast<size_t>(RF_S2) * M + b], A.rowtab[static_cast<size_t>(RF_COS) * M + b],
                      A.rowtab[static_cast<size_t>(RF_G) * M + b], A.rowtab[static_cast<size_t>(RF_CTAN) * M + b]);
+      // The grid scales go into the kept coefficients: the stencils have whole
+      // weights (fewer operations and registers: 1024 x 64 6.1 -> 5.8 us a step).
+      C.ctan /= A.cyy;
+#pragma unroll
+      for (int c = 0; c < COLS; c++) {
+        C.cc[c] *= A.cyy;
+        C.bb[c] *= A.cx;
+        C.ee[c] *= A.cx;
+        C.dre[c] *= A.cx;
+        C.dim[c] *= A.cx;
+      }
     }
     if (ends) {
       close_ends(q0 + (3 + r) * WC, qpl);
@@ -321,8 +332,13 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
     if (A.hist != nullptr && A.ext[e] >= a0 && A.ext[e] < a0 + COLS) hist_col = 2 * (A.ext[e] - a0) + e;
   const bool hist_both = COLS == 2 && A.hist != nullptr && A.ext[0] >= a0 && A.ext[0] < a0 + COLS && A.ext[1] >= a0 && A.ext[1] < a0 + COLS;
 
+  // Stencil weights, with the grid scales where the coefficients lack them.
   const double d1a = 45.0 * A.cx, d1b = -9.0 * A.cx, d1c_ = A.cx;
   const double y2a = -490.0 * A.cyy, y2b = 270.0 * A.cyy, y2c = -27.0 * A.cyy, y2d = 2.0 * A.cyy;
+  auto d1 = [&](const double (&v)[8 + COLS], const int c) {
+    return KEEP ? fma(45.0, v[5 + c] - v[3 + c], fma(-9.0, v[6 + c] - v[2 + c], v[7 + c] - v[1 + c]))
+                : fma(d1a, v[5 + c] - v[3 + c], fma(d1b, v[6 + c] - v[2 + c], d1c_ * (v[7 + c] - v[1 + c])));
+  };
   const double pole_w = A.even_m ? kThird : 0.0;
   // cq f + cu u, with the terms the weights (constants once unrolled) take out left out.
   auto combine = [](const double cq, const double f, const double cu, const double u) {
@@ -417,11 +433,13 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
           for (int c = 0; c < COLS; c++) {
             // Theta derivatives (HighOrder/kern.cu:206-226).
             const double y1 = fma(45.0, g[4][c] - g[2][c], fma(-9.0, g[5][c] - g[1][c], g[6][c] - g[0][c]));
-            const double y2 = fma(y2a, g[3][c], y2b * (g[4][c] + g[2][c])) +
-                              fma(y2c, g[5][c] + g[1][c], y2d * (g[6][c] + g[0][c]));
+            const double y2 = KEEP ? fma(-490.0, g[3][c], 270.0 * (g[4][c] + g[2][c])) +
+                                         fma(-27.0, g[5][c] + g[1][c], 2.0 * (g[6][c] + g[0][c]))
+                                   : fma(y2a, g[3][c], y2b * (g[4][c] + g[2][c])) +
+                                         fma(y2c, g[5][c] + g[1][c], y2d * (g[6][c] + g[0][c]));
             const double ll = fma(C.ctan, y1, y2), f = v[4 + c];
             // Radial derivative and dissipation (HighOrder/kern.cu:233-261).
-            const double fx = fma(d1a, v[5 + c] - v[3 + c], fma(d1b, v[6 + c] - v[2 + c], d1c_ * (v[7 + c] - v[1 + c])));
+            const double fx = d1(v, c);
             const double kd = fma(-8.0, v[7 + c] + v[1 + c], v[8 + c] + v[c]) +
                               fma(28.0, v[6 + c] + v[2 + c], fma(-56.0, v[5 + c] + v[3 + c], 70.0 * f));
             o[pl][c] = fma(cr, fma(kon[c], kd, fma(-C.bb[c], fx, pc[pl][c])), combine(cq, f, cu, u[c]));
@@ -503,7 +521,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
           get<COLS>(u, us + ((2 + pl) * RS + r) * TC + col);
 #pragma unroll
           for (int c = 0; c < COLS; c++) {
-            const double fx = fma(d1a, v[5 + c] - v[3 + c], fma(d1b, v[6 + c] - v[2 + c], d1c_ * (v[7 + c] - v[1 + c])));
+            const double fx = d1(v, c);
             const double kd = fma(-8.0, v[7 + c] + v[1 + c], v[8 + c] + v[c]) +
                               fma(28.0, v[6 + c] + v[2 + c], fma(-56.0, v[5 + c] + v[3 + c], 70.0 * v[4 + c]));
             const double t = pl == 0 ? fma(C.are[c], pc[0][c], fma(-C.aim[c], pc[1][c], res[0][c]))
