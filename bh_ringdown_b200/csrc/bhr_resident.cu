@@ -186,6 +186,19 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
   const int col = COLS == 2 ? 2 * lane : 32 * (warp & 1) + lane;        // this thread's first column in the tile
   const int a0 = c0 + col, w0 = col + 4;
 
+  // Stencil weights, with the grid scales where the coefficients lack them.
+  const double d1a = 45.0 * A.cx, d1b = -9.0 * A.cx, d1c_ = A.cx;
+  const double y2a = __dmul_rn(-490.0, A.cyy), y2b = __dmul_rn(270.0, A.cyy), y2c = __dmul_rn(-27.0, A.cyy),
+               y2d = __dmul_rn(2.0, A.cyy);
+  // The second derivative's scaled weights do not add up to zero as whole ones
+  // do.  What is left of their sum (formed here without rounding) acts on f
+  // itself, always the same way: it is taken out of the p equation's
+  // coefficient of f, with RF_G.  Left in, the error against 80 bits grows past
+  // that of the stage launches with the step count (896 x 176 1.87 times as
+  // large after 120 steps, 1024 x 176 4.7 times after 332; without it 0.9).
+  // Whole weights instead cost 4-5 % of a step (more spills).
+  const double y2_rest = KEEP ? 0.0 : 2.0 * (0.5 * y2a + y2b + y2c + y2d);
+
   // ---- the tile: state with its halo, and what the coefficients are made of
   if (tid == 0) abort_flag = 0;
   for (int i = tid; i < 2 * (R + 6) * (WC / 2); i += kResThreads) {
@@ -204,8 +217,10 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
     *reinterpret_cast<double2 *>((pl < 2 ? p0 + pl * ppl : bbs) + j * WC + w) = v;
   }
   if (!KEEP) {
-    for (int i = tid; i < R * RF_COUNT; i += kResThreads)
-      rowf[i] = A.rowtab[static_cast<size_t>(i % RF_COUNT) * M + b0 + i / RF_COUNT];
+    for (int i = tid; i < R * RF_COUNT; i += kResThreads) {
+      const double v = A.rowtab[static_cast<size_t>(i % RF_COUNT) * M + b0 + i / RF_COUNT];
+      rowf[i] = i % RF_COUNT == RF_G ? v + y2_rest : v;
+    }
     for (int i = tid; i < CF_TILE * TC; i += kResThreads) colf[i] = A.coltab[static_cast<size_t>(i / TC) * N + c0 + i % TC];
   }
   // Stored columns, and the weight of the Kreiss-Oliger term.
@@ -332,9 +347,6 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
     if (A.hist != nullptr && A.ext[e] >= a0 && A.ext[e] < a0 + COLS) hist_col = 2 * (A.ext[e] - a0) + e;
   const bool hist_both = COLS == 2 && A.hist != nullptr && A.ext[0] >= a0 && A.ext[0] < a0 + COLS && A.ext[1] >= a0 && A.ext[1] < a0 + COLS;
 
-  // Stencil weights, with the grid scales where the coefficients lack them.
-  const double d1a = 45.0 * A.cx, d1b = -9.0 * A.cx, d1c_ = A.cx;
-  const double y2a = -490.0 * A.cyy, y2b = 270.0 * A.cyy, y2c = -27.0 * A.cyy, y2d = 2.0 * A.cyy;
   auto d1 = [&](const double (&v)[8 + COLS], const int c) {
     return KEEP ? fma(45.0, v[5 + c] - v[3 + c], fma(-9.0, v[6 + c] - v[2 + c], v[7 + c] - v[1 + c]))
                 : fma(d1a, v[5 + c] - v[3 + c], fma(d1b, v[6 + c] - v[2 + c], d1c_ * (v[7 + c] - v[1 + c])));
