@@ -352,10 +352,6 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
                 : fma(d1a, v[5 + c] - v[3 + c], fma(d1b, v[6 + c] - v[2 + c], d1c_ * (v[7 + c] - v[1 + c])));
   };
   const double pole_w = A.even_m ? kThird : 0.0;
-  // cq f + cu u, with the terms the weights (constants once unrolled) take out left out.
-  auto combine = [](const double cq, const double f, const double cu, const double u) {
-    return cu == 0.0 ? f : cq == 0.0 ? u : cu == 1.0 ? fma(cq, f, u) : fma(cq, f, cu * u);
-  };
   unsigned long long seq = A.seq;
   bool aborted = false, first = true;
   int cur = 0;  // buffer of the stage input
@@ -379,13 +375,20 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
       const double *q = q0 + cur * 2 * qpl;
       double *qn = q0 + (cur ^ 1) * 2 * qpl;
       double *p = p0 + (PBUFS == 2 ? cur * 2 * ppl : 0), *pn = p0 + (PBUFS == 2 ? (cur ^ 1) * 2 * ppl : 0);
-      // The stage combination cu u^n + cq f + cr L (HighOrder/kern.cu:
-      // 301-318, 582-620; the weights as the reference rounds them).  RK4:
-      // u + dt/2 L, u + dt/2 L, u + dt L, z + y3/3 + dt/6 L.
-      const double cu = RK4 ? (stage == 1 ? 0.0 : 1.0) : stage == 1 ? 0.0 : stage == 2 ? 0.75 : kThird;
-      const double cq = RK4 ? (stage == 1 ? 1.0 : stage == 4 ? kThird : 0.0)
-                            : stage == 1 ? 1.0 : stage == 2 ? 0.25 : 2.0 * kThird;
-      const double cr = RK4 ? (stage < 3 ? 0.5 * A.dt : stage == 3 ? A.dt : A.dt / 6.0) : cq * A.dt;
+      // The stage combination, f + dt L, (3 u^n + f + dt L)/4 and (u^n + 2 f +
+      // 2 dt L)/3 (HighOrder/kern.cu:301-318, 582-620), rounded as these forms
+      // round: where f = u^n the first two terms come out as u^n.  With the
+      // weights 3/4, 1/4, 1/3 and 2/3 on the terms one by one (the last two
+      // rounded down) they do not, and the waveform drifts: 1024 x 64 after
+      // 2500 steps 8.7e-15 from the stage launches', like this 3.8e-16.
+      // RK4: u^n + dt/2 L, u^n + dt/2 L, u^n + dt L, z + y3/3 + dt/6 L.
+      const double cr = RK4 ? (stage < 3 ? 0.5 * A.dt : stage == 3 ? A.dt : A.dt / 6.0)
+                            : stage == 1 ? A.dt : stage == 2 ? 0.25 * A.dt : 2.0 * kThird * A.dt;
+      auto terms = [&](const double f, const double u) {
+        if (stage == 1) return f;
+        if (RK4) return stage == 4 ? fma(kThird, f, u) : u;
+        return stage == 2 ? fma(0.75, u, 0.25 * f) : kThird * fma(2.0, f, u);
+      };
       const double *us = RK4 && stage == 4 ? zn : un;
 #pragma unroll 1
       for (int i = 0; i < RPW; i++) {
@@ -454,7 +457,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
             const double fx = d1(v, c);
             const double kd = fma(-8.0, v[7 + c] + v[1 + c], v[8 + c] + v[c]) +
                               fma(28.0, v[6 + c] + v[2 + c], fma(-56.0, v[5 + c] + v[3 + c], 70.0 * f));
-            o[pl][c] = fma(cr, fma(kon[c], kd, fma(-C.bb[c], fx, pc[pl][c])), combine(cq, f, cu, u[c]));
+            o[pl][c] = fma(cr, fma(kon[c], kd, fma(-C.bb[c], fx, pc[pl][c])), terms(f, u[c]));
             if (RK4 && stage == 2) zn[(pl * RS + r) * TC + col + c] = (f + 2.0 * o[pl][c] - u[c]) * kThird;
             // the p equation's q terms (HighOrder/kern.cu:281-296)
             if (pl == 0) {
@@ -539,7 +542,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
             const double t = pl == 0 ? fma(C.are[c], pc[0][c], fma(-C.aim[c], pc[1][c], res[0][c]))
                                      : fma(C.are[c], pc[1][c], fma(C.aim[c], pc[0][c], res[1][c]));
             const double x = SRC ? t + sv[pl][c] : t;
-            o[pl][c] = fma(cr, fma(C.ee[c], fx, fma(kon[c], kd, x)), combine(cq, v[4 + c], cu, u[c]));
+            o[pl][c] = fma(cr, fma(C.ee[c], fx, fma(kon[c], kd, x)), terms(v[4 + c], u[c]));
             if (RK4 && stage == 2) zn[((2 + pl) * RS + r) * TC + col + c] = (v[4 + c] + 2.0 * o[pl][c] - u[c]) * kThird;
           }
         }

@@ -4,7 +4,8 @@ way in every stage.
 
 Bounds, with n stages: fields 8 sqrt(n) 2^-53 of their norm -- a random walk
 of 64 roundings a stage, the terms of an update that are as large as the field
-itself or larger (dissipation, second derivative)."""
+itself or larger (dissipation, second derivative); waveforms, integrals over
+the theta of many points, sqrt(n) 2^-53, the walk of one rounding a stage."""
 import numpy as np
 import pytest
 
@@ -31,3 +32,11 @@ def test_fields_of_two_row_tiles_drift_by_rounding_only(a, m, monkeypatch):
     (u, _), (v, _) = (evolve(896, 176, a, m, steps, tl, monkeypatch) for tl in ("resident", "block8n"))
     bound = 8.0 * np.sqrt(3 * steps) * 2.0 ** -53
     assert np.linalg.norm(u - v) <= bound * np.linalg.norm(v)
+
+
+@pytest.mark.parametrize("N,M,a,m", [(896, 176, 0.7, 2), (896, 176, 0.9, 3), (1216, 80, 0.7, 2), (1216, 80, 0.3, -1)])
+def test_waveforms_drift_by_rounding_only(N, M, a, m, monkeypatch):
+    steps = 5000
+    (_, (t, h, _)), (_, (t1, h1, _)) = (evolve(N, M, a, m, steps, tl, monkeypatch) for tl in ("resident", "block8n"))
+    assert np.array_equal(t, t1)
+    assert np.linalg.norm(h - h1) <= np.sqrt(3 * steps) * 2.0 ** -53 * np.linalg.norm(h1)
