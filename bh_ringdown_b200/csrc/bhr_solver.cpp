@@ -169,7 +169,6 @@ static int autotune_rows(bhr_solver *s);
 static bool runs_resident(const bhr_solver *s);
 static int late_dependents(int blocks, int next, int per_sm);
 static void history_columns(const bhr_solver *s, int ext[2]);
-static cudaError_t launch_sources_ahead(bhr_solver *s, int done);
 
 extern "C" {
 
@@ -807,10 +806,10 @@ int bhr_solver_set_trajectory(bhr_solver *s, const double *rows, int nrows) {
       return BHR_OUT_OF_MEMORY;
     }
   }
-  // The patches of the first sequence (later ones are built beside the stages).
+  // No patch of these records is there.  None is built here: only the first
+  // kFirstRecords records are (and the trajectory may be set at any step);
+  // enqueue_steps builds patches once it has waited for theirs.
   s->built = 0;
-  if (!runs_resident(s)) BHR_CUDA_TRY(launch_sources_ahead(s, s->steps_done));
-  BHR_CUDA_TRY(cudaStreamSynchronize(s->stream));
   // The launch arguments now carry the source and the new records: step
   // graphs captured before (steps taken without a trajectory) are rebuilt.
   if (s->g1) cudaGraphExecDestroy(s->g1);
