@@ -136,7 +136,7 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
   const bool rebuild = !same_tables(D, *p);
   const ResidentGeom geom = resident_geometry(N, M);
   bool resident = geom.ok && resident_inbox_bytes(geom) <= 2 * kStageDoubles * sizeof(double);
-  auto encode = [&]() -> int {
+  auto encode = [&] {
     for (int i = 0; i < 3; i++) {
       double *bufs[3] = {state, u1, u2};
       StageMaps &mp = D.maps[i];
@@ -146,11 +146,11 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
           encode_state_maps(bufs[i], N, M, TR, &mp.q, &mp.p, nullptr) != cudaSuccess ||
           encode_coef_maps(ctab, coltab, rowtab, N, M, TR, &mp) != cudaSuccess) {
         D.state = nullptr;
-        return fail(BHR_CUDA_ERROR, "bhr_step_noalloc: cuTensorMapEncodeTiled failed");
+        return false;
       }
     }
     D.state = state;
-    return BHR_OK;
+    return true;
   };
   if (rebuild) {
     // The tables are rewritten while no kernel of an earlier call may still
@@ -251,8 +251,7 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
     }
   }
   if (!resident) {
-    if (D.state != state)
-      if (int rc = encode()) return rc;
+    if (D.state != state && !encode()) failed = "bhr_step_noalloc: cuTensorMapEncodeTiled failed";
     D.inbox_valid = false;  // u1 and u2 hold stages from here on
   }
   // The stage kernels request the coefficient tiles before their grid-
