@@ -272,6 +272,7 @@ extern "C" int bhr_step_noalloc(const bhr_params *p, double *state, int nsteps, 
     // call may rewrite the tables these kernels read.
     cudaStreamSynchronize(st);
     cudaGetLastError();
+    D.flag_clear = false;  // the launches before the one that failed may have set it
     return fail(BHR_CUDA_ERROR, failed);
   }
   int h_flag = 0;

@@ -105,5 +105,14 @@ int main() {
   check(step(p, 3) == BHR_OK && has("resident") && !has("stage") && !has("old seq"), "resident again");
   check(find("clear words") >= 0 && find("clear words") < find("resident"), "stages are cleared out of the edge words");
   check(step(p, 3) == BHR_OK && has("resident") && !has("clear words") && !has("old seq"), "the words are kept from call to call");
+
+  // The first launch of a long call may have set the error flag before the
+  // second one failed: the next call clears it.
+  check(!has("clear flag"), "the flag is not cleared after calls that ended well");
+  fail_resident_at = 1, resident_error = cudaErrorLaunchFailure;
+  check(step(p, 5000) == BHR_CUDA_ERROR && resident_launches == 2 && undrained == 0, "the second launch fails");
+  fail_resident_at = -1;
+  check(step(p, 1) == BHR_OK && find("clear flag") >= 0 && find("clear flag") < find("resident"),
+        "the call after a failed one clears the flag");
   return failures != 0;
 }
