@@ -320,7 +320,8 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
 
   const size_t NM = static_cast<size_t>(p.N) * p.M;
   int st = BHR_OK;
-  // Patch buffers: this sequence's and the next one's steps, two at least.
+  // Patch buffers: this sequence's and the next one's steps, two at least
+  // (set_trajectory allocates them: 8 to 16 MB that source-free solves do without).
   const size_t patch = 2 * static_cast<size_t>(p.PTSX) * p.PTSY;
   const bool engine = tile_rows != 0;  // which steps its solves one by one
   // Not the batch engine's solves, whose tile height the caller fixes, nor
@@ -350,7 +351,7 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
       (st = dalloc(s, &s->coltab, static_cast<size_t>(CF_COUNT) * p.N)) ||
       (st = dalloc(s, &s->rowtab, static_cast<size_t>(RF_COUNT) * p.M)) || (st = dalloc(s, &s->ctab, NM)) ||
       (st = dalloc(s, &s->rc, p.N)) ||
-      (st = dalloc(s, &s->th, p.M)) || (st = dalloc(s, &s->src, s->nbuf * patch)) ||
+      (st = dalloc(s, &s->th, p.M)) ||
       (st = dalloc(s, &s->ext, 2 * static_cast<size_t>(p.M))) || (st = dalloc(s, &s->integ, 4 * static_cast<size_t>(p.M))) ||
       (st = dalloc(s, &s->wproj, 7 * static_cast<size_t>(p.M))) || (st = dalloc(s, &s->wdedt, p.M)) ||
       (st = dalloc(s, &s->rows, 16 * static_cast<size_t>(s->max_rows))) ||
@@ -381,7 +382,6 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
       (e = launch_coef_tables(s->coltab, s->rowtab, s->ctab, p.N, p.M, s->stream)) ||
       (e = cudaMemsetAsync(s->u1, 0, 4 * NM * 8, s->stream)) || (e = cudaMemsetAsync(s->u2, 0, 4 * NM * 8, s->stream)) ||
       (e = cudaMemsetAsync(s->integ, 0, 4 * p.M * 8, s->stream)) || (e = cudaMemsetAsync(s->ext, 0, 2 * p.M * 8, s->stream)) ||
-      (e = cudaMemsetAsync(s->src, 0, s->nbuf * patch * 8, s->stream)) ||
       (e = cudaMemsetAsync(s->rs, 0, sizeof(RunState), s->stream)) || (e = cudaStreamSynchronize(s->stream))) {
     set_error(std::string("upload: ") + cudaGetErrorString(e));
     if (dfac) cudaFreeAsync(dfac, s->stream);
@@ -781,6 +781,11 @@ int bhr_solver_set_trajectory(bhr_solver *s, const double *rows, int nrows) {
     return bad_status;
   }
   cudaSetDevice(p.device);
+  if (!s->src) {
+    const size_t n = 2 * static_cast<size_t>(s->nbuf) * p.PTSX * p.PTSY;
+    if (int st = dalloc(s, &s->src, n)) return st;
+    BHR_CUDA_TRY(cudaMemsetAsync(s->src, 0, n * 8, s->stream));
+  }
   if (s->recs) cudaFreeAsync(s->recs, s->stream), s->bytes -= sizeof(StepRec) * static_cast<size_t>(s->nt ? s->nt : 1);
   s->recs = nullptr;
   if (int st = dalloc(s, &s->recs, static_cast<size_t>(s->nt))) return st;
