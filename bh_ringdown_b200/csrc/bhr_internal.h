@@ -70,9 +70,17 @@ enum StageDir { kSameWay = 0, kForward = 1, kBackward = 2 };
 // Steps a solve's history holds: those of two sequences.
 constexpr int kHistSteps = 32;
 // Bytes of states (one solve's, or a batch's) from which on consecutive
-// stages walk the tiles in opposite directions.
-constexpr size_t kTurnBytes = 96u << 20;
-constexpr size_t kTurnMixedBytes = 128u << 20;  // the FP32 stages of mixed precision (of its FP64 states)
+// stages walk the tiles in opposite directions: shares of the device's L2
+// (132.6 MB), between measured sizes.  us a step, same way and in turn:
+// SSP-RK3 8192 x 96 (75.5 MB) 45.7 and 45.7, 7168 x 112 (77.1) 46.7 and 46.5,
+// 8192 x 112 (88.1) 53.1 and 52.4, 8192 x 128 60.7 and 58.7, 16384 x 128 106
+// and 103; RK4, of four states, 4096 x 144 (75.5 MB) 51.4 and 51.4, 4096 x 160
+// (83.9) 58.2 and 57.3, 8192 x 128 88.6 and 83.5.
+constexpr size_t turn_bytes(size_t l2) { return l2 / 5 * 3; }
+// The FP32 stages of mixed precision, by its FP64 states (same way and in
+// turn, the FP64 stage turning): 8192 x 128 (100.7 MB) 51.3 and 51.6, 8192 x 144
+// (113.2) 56.1 and 55.8, 8192 x 160 61.9 and 60.5, 8192 x 192 72.3 and 70.5.
+constexpr size_t turn_mixed_bytes(size_t l2) { return l2 / 5 * 4; }
 
 struct StageArgs {
   const double *vin;    // stage input planes (also the TMA source)
@@ -334,5 +342,7 @@ cudaError_t prepare_kernels();
 int stage_prefetch_ahead(int requested = -1);
 // The device's SM count (cached per device).
 int device_sm_count();
+// The current device's L2.
+size_t device_l2_bytes();
 
 }  // namespace bhr

@@ -1520,6 +1520,12 @@ int stage_prefetch_ahead(const int requested) {
   return requested >= 0 ? requested : 2 * sm_count();
 }
 int device_sm_count() { return sm_count(); }
+size_t device_l2_bytes() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrL2CacheSize, dev) != cudaSuccess || n <= 0)
+    return 126u << 20;
+  return static_cast<size_t>(n);
+}
 
 cudaError_t launch_stage(int stage, const StageMaps &maps, const StageArgs &a_in, cudaStream_t st, bool pdl) {
   StageArgs a = a_in;

@@ -347,6 +347,7 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
     delete s;
     return BHR_CUDA_ERROR;
   }
+  s->l2 = device_l2_bytes();
   if ((st = dalloc(s, &s->u0, 4 * NM)) || (st = dalloc(s, &s->u1, 4 * NM)) || (st = dalloc(s, &s->u2, 4 * NM)) ||
       (st = dalloc(s, &s->coltab, static_cast<size_t>(CF_COUNT) * p.N)) ||
       (st = dalloc(s, &s->rowtab, static_cast<size_t>(RF_COUNT) * p.M)) || (st = dalloc(s, &s->ctab, NM)) ||
@@ -1090,18 +1091,17 @@ ExtractArgs bhr::solver_extract_args(bhr_solver *s) {
   return E;
 }
 
-// Solves whose states take kTurnBytes and more are walked back and forth.
-// Measured (us per step, same way -> in turn): 8192 x 128 63.0 -> 62.2 (100 MB
-// of states), 16000 x 256 201 -> 197, 16384 x 256 plunge 204 -> 200; below,
-// where L2 holds the states in any order, nothing is gained and the last
+// Solves whose states do not stay in L2 are walked back and forth (turn_bytes;
+// us per step, same way -> in turn: 16000 x 256 201 -> 197, 16384 x 256 plunge
+// 204 -> 200); where L2 holds them in any order, nothing is gained and the last
 // blocks' prefetch of the next stage's first tiles would be lost.  Mixed
 // precision: the FP64 stage begins forward and backward from step to step
-// (8192 x 128 53.4 -> 52.5, 8192 x 160 63.9 -> 62.5), the FP32 stages turn with
-// it from kTurnMixedBytes on (8192 x 128 53.4 with them, 8192 x 192 73.0 -> 70.9).
+// (8192 x 128 52.1 -> 51.3, 8192 x 160 63.5 -> 61.9), the FP32 stages turn with
+// it from turn_mixed_bytes on.
 static size_t state_bytes(const bhr_solver *s) {
   return (s->rk4 ? 4 : 3) * sizeof(double) * 4 * static_cast<size_t>(s->p.N) * s->p.M;
 }
-static bool solver_turns(const bhr_solver *s) { return s->narrow && !s->strip12 && state_bytes(s) >= kTurnBytes; }
+static bool solver_turns(const bhr_solver *s) { return s->narrow && !s->strip12 && state_bytes(s) >= turn_bytes(s->l2); }
 
 // The columns a step's history keeps: the extraction column, or the two
 // interior ones its closure is made of.
@@ -1135,7 +1135,7 @@ static int launch_stages(bhr_solver *s, int step, bool record, bool flip, cudaEv
   StageArgs A = solver_stage_args(s);
   A.step = step;
   // Consecutive stages walk the grid in opposite directions where the states
-  // do not stay in L2 (kTurnBytes), so each starts on the tiles the one before
+  // do not stay in L2 (turn_bytes), so each starts on the tiles the one before
   // wrote last.
   const StageBlocks B(s);
   A.late = B.one_tile && late_dependents(B.stage, B.stage, B.per_sm);
@@ -1168,7 +1168,7 @@ static int launch_stages(bhr_solver *s, int step, bool record, bool flip, cudaEv
     MixedArgs X = solver_mixed_args(s);
     X.e_out = s->e2f;
     X.late = late_dependents(B.mixed, B.mixed, B.mixed_per_sm);
-    const bool turn32 = turns && state_bytes(s) >= kTurnMixedBytes;
+    const bool turn32 = turns && state_bytes(s) >= turn_mixed_bytes(s->l2);
     BHR_CUDA_TRY(launch_mixed_stage(2, s->mmaps[0], X, turn32 && !flip, s->stream));
     BHR_CUDA_TRY(mark(2));
     X.e_out = nullptr;

@@ -58,6 +58,7 @@ struct bhr_solver {
   bhr::ResidentGeom rgeom{};
   ulonglong2 *inbox = nullptr;   // edge words of the blocks
   unsigned long long rseq = 1;   // number of the next launch's first edge words
+  size_t l2 = 0;       // bytes of the device's L2
   int steps_done = 0;
   int nbuf = 2;        // source patch buffers
   int built = 0;       // the patches of the steps up to this one, from steps_done on, are there (by stage)
