@@ -315,7 +315,7 @@ int rebuild(bhr_engine *e) {
   // 183.3 ms in all, without 180).  Others: capture one batch step.
   size_t state_bytes = 0;
   for (const Running &R : e->active) state_bytes += 3 * sizeof(double) * 4 * static_cast<size_t>(R.s->p.N) * R.s->p.M;
-  if (state_bytes >= turn_bytes(device_l2_bytes())) return BHR_OK;
+  if (batch_turns(e->tiling, state_bytes, device_l2_bytes())) return BHR_OK;
   cudaGraph_t g = nullptr;
   if ((err = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal)))
     return set_fail(BHR_CUDA_ERROR, std::string("capture: ") + cudaGetErrorString(err));

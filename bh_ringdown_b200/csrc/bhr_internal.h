@@ -323,6 +323,10 @@ constexpr int tiling_rows(int tiling) {
 }
 // Tile height of the mixed-precision FP32 stage kernels.
 constexpr int kMixTileRows = 16;
+// Whether a batch's steps turn: only the block8n kernels take a direction.
+constexpr bool batch_turns(int tiling, size_t states, size_t l2) {
+  return tiling == kTilingBlock8n && states >= turn_bytes(l2);
+}
 // One launch of an FP64 stage over a group of a batch's solves (tiles of the
 // tiling's height).
 cudaError_t launch_stage_batch(int stage, int tiling, const BatchSolve *solves, const BatchGroup &g, bool backward,

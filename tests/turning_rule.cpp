@@ -21,5 +21,9 @@ int main() {
         "the FP32 stages turn from 8192 x 144 on");
   check(turn_bytes(2 * l2) >= 2 * turn_bytes(l2) && turn_mixed_bytes(2 * l2) >= 2 * turn_mixed_bytes(l2),
         "the sizes grow with the L2");
+  for (int tiling : {kTilingBlock8, kTilingBlock16, kTilingPersistent, kTilingRing})
+    check(!batch_turns(tiling, states(3, 16384, 256), l2), "batches whose kernels take no direction keep their graph");
+  check(batch_turns(kTilingBlock8n, states(3, 8192, 112), l2) && !batch_turns(kTilingBlock8n, states(3, 8192, 96), l2),
+        "batches of block8n tiles turn from the same size on as single solves");
   return failures != 0;
 }
