@@ -341,11 +341,12 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
     T.pole = b < 6 || b >= M - 6;
   };
   if (KEEP) targets(row0);
-  int hist_col = -1;  // this thread holds extraction column hist_col & 1 in its column hist_col >> 1
+  // This thread holds extraction column hist_col & 1 in its column hist_col >>
+  // 1 (never both: of 3, 4 and of N - 4, N - 5 each lies in another pair).
+  int hist_col = -1;
 #pragma unroll
   for (int e = 0; e < 2; e++)
     if (A.hist != nullptr && A.ext[e] >= a0 && A.ext[e] < a0 + COLS) hist_col = 2 * (A.ext[e] - a0) + e;
-  const bool hist_both = COLS == 2 && A.hist != nullptr && A.ext[0] >= a0 && A.ext[0] < a0 + COLS && A.ext[1] >= a0 && A.ext[1] < a0 + COLS;
 
   auto d1 = [&](const double (&v)[8 + COLS], const int c) {
     return KEEP ? fma(45.0, v[5 + c] - v[3 + c], fma(-9.0, v[6 + c] - v[2 + c], v[7 + c] - v[1 + c]))
@@ -500,19 +501,11 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
             }
           }
           if (hist_col >= 0) {
-            // psi at the extraction column (or the two its closure is made of)
-            double *h = A.hist + static_cast<size_t>(4 * step) * M + b;
-            const int e = hist_col & 1;
-#pragma unroll
-            for (int c = 0; c < COLS; c++) {
-              if (hist_col >> 1 == c) {
-                h[2 * e * M] = o[0][c];
-                h[(2 * e + 1) * M] = o[1][c];
-              } else if (hist_both) {
-                h[2 * (e ^ 1) * M] = o[0][c];
-                h[(2 * (e ^ 1) + 1) * M] = o[1][c];
-              }
-            }
+            // psi at the extraction column (or one of the two its closure is made of)
+            double *h = A.hist + static_cast<size_t>(4 * step + 2 * (hist_col & 1)) * M + b;
+            const bool second = COLS == 2 && hist_col >= 2;
+            h[0] = second ? o[0][COLS - 1] : o[0][0];
+            h[M] = second ? o[1][COLS - 1] : o[1][0];
           }
         }
         if (ends) close_ends(qn + (3 + r) * WC, qpl);
