@@ -304,6 +304,8 @@ cudaError_t launch_coef_tables(const double *coltab, const double *rowtab, doubl
                                cudaStream_t st);
 cudaError_t encode_coef_maps(double *ctab, const double *coltab, const double *rowtab, int N, int M, int rows,
                              StageMaps *maps);
+// Whether a patch of that width can be built (a block has a thread per column).
+cudaError_t source_launchable(int PTSX);
 // The patches of count steps from rs->ks + lookahead on.
 cudaError_t launch_source(const SourceArgs &a, int count, cudaStream_t st);
 // persist = 1 walks the work-list with one block per SM (16-row tiles);

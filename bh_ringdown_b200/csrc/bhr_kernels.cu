@@ -1668,6 +1668,12 @@ cudaError_t launch_extract_batch(const ExtractArgs *args, int nsolves, cudaStrea
   return launch_pdl(extract_batch_kernel, dim3(nsolves), dim3(kExtractThreads), 0, st, args);
 }
 
+cudaError_t source_launchable(int PTSX) {
+  cudaFuncAttributes at{};
+  if (cudaError_t e = cudaFuncGetAttributes(&at, source_patch_kernel)) return e;
+  return std::max(PTSX, kSrcRows) <= at.maxThreadsPerBlock ? cudaSuccess : cudaErrorLaunchOutOfResources;
+}
+
 cudaError_t launch_source(const SourceArgs &a, int count, cudaStream_t st) {
   return launch_pdl(source_patch_kernel, dim3((a.PTSY + kSrcRows - 1) / kSrcRows, count),
                     dim3(std::max(a.PTSX, kSrcRows)), 0, st, a);

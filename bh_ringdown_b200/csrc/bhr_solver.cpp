@@ -816,6 +816,7 @@ int bhr_solver_set_trajectory(bhr_solver *s, const double *rows, int nrows) {
   // kFirstRecords records are (and the trajectory may be set at any step);
   // enqueue_steps builds patches once it has waited for theirs.
   s->built = 0;
+  BHR_CUDA_TRY(source_launchable(p.PTSX));
   // The launch arguments now carry the source and the new records: step
   // graphs captured before (steps taken without a trajectory) are rebuilt.
   if (s->g1) cudaGraphExecDestroy(s->g1);
