@@ -61,8 +61,12 @@ static constexpr size_t kDirectPoints = 400000;
 // and extraction are 14 us (8192 x 128, wall us of two steps: 141 one by one, 158
 // as a sequence; of four 269 and 279, of five 345 and 337).
 static constexpr int kFewSteps = 4;
-// Patch buffers of a solve take at most this much (two at least).
+// Patch buffers of a solve take at most this much, but there are those of two
+// sequences of four steps: with two buffers sources are built between the steps,
+// not beside them (us a step, two buffers, four and eight: 8192 x 128 with patches
+// of 700 x 1600 76.8, 75.5 and 73.9, of 800 x 3000 89.9, 86.5 and 84.2).
 static constexpr size_t kPatchBytes = 64u << 20;
+static constexpr int kLeastSequence = 4;
 
 namespace {
 
@@ -320,8 +324,8 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
 
   const size_t NM = static_cast<size_t>(p.N) * p.M;
   int st = BHR_OK;
-  // Patch buffers: this sequence's and the next one's steps, two at least
-  // (set_trajectory allocates them: 8 to 16 MB that source-free solves do without).
+  // Patch buffers: this sequence's and the next one's steps (set_trajectory
+  // allocates them: 8 MB and more that source-free solves do without).
   const size_t patch = 2 * static_cast<size_t>(p.PTSX) * p.PTSY;
   const bool engine = tile_rows != 0;  // which steps its solves one by one
   // Not the batch engine's solves, whose tile height the caller fixes, nor
@@ -332,7 +336,9 @@ int bhr::solver_create(const bhr_params *pin, int tile_rows, bhr_solver **out) {
     s->resident = s->rgeom.ok;
   }
   const int sequences = s->resident && s->rgeom.rmax <= kResidentSourceRows ? kResidentChunk / 2 : kSequence;
-  s->nbuf = engine ? 2 : 2 * static_cast<int>(std::max<size_t>(1, std::min<size_t>(sequences, kPatchBytes / (16 * patch))));
+  s->nbuf = 2;
+  if (!engine)
+    s->nbuf *= std::max(kLeastSequence, static_cast<int>(std::min<size_t>(sequences, kPatchBytes / (16 * patch))));
   // The side stream (sources, extraction: a few blocks beside the stages)
   // gets the device's highest priority, so its blocks take the first SM
   // slots that free up.
@@ -1397,10 +1403,10 @@ static bool call_is_resident(const bhr_solver *s, int nsteps) {
 // steps, of a full sequence for long runs.
 static int prepare_graphs(bhr_solver *s, int nsteps) {
   if (call_is_resident(s, nsteps)) return BHR_OK;
-  if (nsteps <= kFewSteps && !s->g1) return capture_sequence(s, 1, &s->g1);
+  if (nsteps <= kFewSteps) return s->g1 ? BHR_OK : capture_sequence(s, 1, &s->g1);
   const int length = sequence_length(s);
   const bool graph = s->nt - s->steps_done >= kGraphSteps || static_cast<size_t>(s->p.N) * s->p.M < kDirectPoints;
-  if (length > 1 && nsteps >= length && graph && !s->gb)
+  if (nsteps >= length && graph && !s->gb)
     return capture_sequence(s, length, &s->gb);
   return BHR_OK;
 }
