@@ -372,7 +372,8 @@ def run_ours(args, rank, local_rank, world):
             "timing": {"l2": ("flushed (256 MB write) before each timed step, each step timed alone" if resident else
                               f"working set {3 * 32 * N * M / 2**20:.0f} MiB > L2 (126 MiB): "
                               f"{args.steps} steps back to back, no flush"),
-                       "events": "CUDA events on the solver stream around graph-launched steps",
+                       "events": "CUDA events on the solver stream around the steps (single-step graphs when timed alone, else "
+                                 "sequences of up to 16, captured or launched directly)",
                        "stage_tiling": tiling, "prefetch_ahead_blocks": ahead},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,

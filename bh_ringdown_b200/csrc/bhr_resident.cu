@@ -15,12 +15,12 @@
 // the point itself, so a row forms and sends q first and waits for p's halo
 // after that: q's edges travel while p is formed, p's while the next q is.
 //
-// Measured on 148 SMs, us per step (three stages), stage launches -> here:
-// 256 x 32 10.4 -> 5.0, 1024 x 64 12.7 -> 5.8, 2048 x 64 14.8 -> 9.6,
-// 2048 x 96 21.0 -> 19.0, 2048 x 128 23.2 -> 21.3, 4096 x 64 22.7 -> 20.7.
+// Measured on 148 SMs, us per step (three stages), stage launches (block8n) ->
+// here: 256 x 32 11.8 -> 5.1, 1024 x 64 12.7 -> 5.8, 2048 x 64 15.5 -> 9.3,
+// 2048 x 96 18.9 -> 18.4, 2048 x 128 21.3 -> 20.7, 4096 x 64 20.9 -> 19.9.
 // With a source (the patches of a launch's steps are built before it: 0.5 us a
-// step) 512 x 32 13.1 -> 5.5, 1024 x 64 11.7 -> 6.4, 2048 x 64 15.2 -> 10.4;
-// RK4 512 x 32 14.0 -> 6.7, 1024 x 64 15.1 -> 7.4, 1536 x 64 20.1 -> 11.0.
+// step) 512 x 32 12.6 -> 5.5, 1024 x 64 13.5 -> 6.4, 2048 x 64 16.0 -> 10.0;
+// RK4 512 x 32 16.1 -> 6.5, 1024 x 64 18.2 -> 7.3, 1536 x 64 20.6 -> 10.8.
 // Taller tiles with a source lose to the stage launches, which build sources
 // beside the stages (2048 x 128 22.2 there, 23.7 here; 1152 x 256 23.2, 24.1),
 // and RK4's z takes their shared memory: both stop at 16 rows.
@@ -801,6 +801,12 @@ cudaError_t prepare_resident_kernels() {
 // A resident launch holds its SMs until its last block ends, and its blocks
 // wait for one another, so launches of different streams on one device are
 // put one after another (each waits for the event behind the one before).
+// Beside other work no block waits for one that has not begun: the blocks of a
+// cooperative launch start together, when all of them have room (with one SM
+// held by another kernel for 20 ms all started after it, within a microsecond),
+// and nothing that waits to start goes in before them (beside three streams of
+// launches that never leave an SM idle, tiles of 8-30 us, each of eight
+// launches began 30 us after the one before).
 static cudaError_t launch_cooperative(void (*kernel)(const ResidentArgs), const ResidentArgs &a, size_t smem,
                                       cudaStream_t st) {
   struct Last {
