@@ -377,11 +377,12 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const __grid_c
       double *qn = q0 + (cur ^ 1) * 2 * qpl;
       double *p = p0 + (PBUFS == 2 ? cur * 2 * ppl : 0), *pn = p0 + (PBUFS == 2 ? (cur ^ 1) * 2 * ppl : 0);
       // The stage combination, f + dt L, (3 u^n + f + dt L)/4 and (u^n + 2 f +
-      // 2 dt L)/3 (HighOrder/kern.cu:301-318, 582-620), rounded as these forms
-      // round: where f = u^n the first two terms come out as u^n.  With the
-      // weights 3/4, 1/4, 1/3 and 2/3 on the terms one by one (the last two
-      // rounded down) they do not, and the waveform drifts: 1024 x 64 after
-      // 2500 steps 8.7e-15 from the stage launches', like this 3.8e-16.
+      // 2 dt L)/3 (HighOrder/kern.cu:301-318, 582-620), the sums of u^n and f
+      // rounded as in the stage launches.  kThird is less than 1/3, so a third
+      // of a field at rest comes out low by an ulp in one of four values; with
+      // the weights 3/4, 1/4, 1/3 and 2/3 on the terms one by one, in one of
+      // six.  Such a difference adds up: the waveform of 1024 x 64 after 2500
+      // steps was 8.7e-15 from the stage launches', like this 3.8e-16.
       // RK4: u^n + dt/2 L, u^n + dt/2 L, u^n + dt L, z + y3/3 + dt/6 L.
       const double cr = RK4 ? (stage < 3 ? 0.5 * A.dt : stage == 3 ? A.dt : A.dt / 6.0)
                             : stage == 1 ? A.dt : stage == 2 ? 0.25 * A.dt : 2.0 * kThird * A.dt;
